@@ -13,8 +13,9 @@ enum : int {
     DEVERR_COPY_TIMEOUT = 4,   // a bounded wait for a bulk copy gave up
 };
 
+// Aligned to its size, so that a value moves in one 8- or 16-byte access.
 template <typename T>
-struct cplx {
+struct alignas(2 * sizeof(T)) cplx {
     T x, y;
 };
 
