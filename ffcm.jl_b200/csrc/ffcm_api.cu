@@ -24,6 +24,7 @@
 #include "cg.cuh"
 #include "fft.cuh"
 #include "fft_dispatch.cuh"
+#include "fft_mixed.cuh"
 #include "fft_pipe.cuh"
 #include "fft_tma.cuh"
 #include "slab.cuh"
@@ -188,37 +189,94 @@ int derive_T(const double* Ld, double R_cd, double ad, double ratiod, const int3
     return FFCM_OK;
 }
 
-// Radix plan for a complex FFT of length n (radix 8/4/2 first, then odd primes).
-int make_plan(int n, int tw_stride, FftPlan& p) {
-    p.n = n;
-    p.tw_stride = tw_stride;
-    p.nstages = 0;
-    int m = n;
-    auto push = [&](int r) {
-        if (p.nstages >= FFT_MAX_STAGES) return false;
-        p.radix[p.nstages++] = r;
-        return true;
-    };
-    while (m % 8 == 0) { if (!push(8)) return FFCM_ERR_UNSUPPORTED; m /= 8; }
-    while (m % 4 == 0) { if (!push(4)) return FFCM_ERR_UNSUPPORTED; m /= 4; }
-    while (m % 2 == 0) { if (!push(2)) return FFCM_ERR_UNSUPPORTED; m /= 2; }
-    for (int q = 3; m > 1; q += 2) {
-        while (m % q == 0) {
-            if (q > FFT_MAX_GENERIC_RADIX)
-                return fail(FFCM_ERR_UNSUPPORTED,
-                            "grid dimension has a prime factor above " +
-                                std::to_string(FFT_MAX_GENERIC_RADIX) + " (" + std::to_string(q) + ")");
-            if (!push(q)) return FFCM_ERR_UNSUPPORTED;
-            m /= q;
+// Radices of a mixed-radix line of length n (fft_mixed.cuh): the cheapest
+// product of register butterflies and single primes up to MIX_MAX_PRIME, by a
+// model of a stage's cost per value fitted to measured passes (y pass of 240 x
+// 200 x 160 in Float32: radices 20 10: 55 us, 8 5 5: 63, 25 8: 74, 10 5 4: 84;
+// z pass: 16 10: 78, 20 8: 85, 10 4 4: 115). Largest radix first, so that the last
+// one is the smallest. max_last > 0: also the cheapest plan whose last radix
+// is at most max_last, taken when it has no more than one stage more (the z
+// pass then keeps a fused projector stage in registers).
+struct MixSearch {
+    int best[MIX_MAX_STAGES], cur[MIX_MAX_STAGES];
+    int nbest = 0;
+    double cost = 1e30;
+    bool (*held)(int R);   // radices with a register butterfly
+    double radix_cost(int R) const {
+        // the exchange, address and twiddle work of a stage, and a term for the
+        // threads a wide butterfly's registers leave an SM
+        double c = 6.0 + 0.01 * R * R;
+        for (int q = 2, m = R; m > 1; ++q)
+            while (m % q == 0) {
+                c += q == 2 ? 1.0 : q == 3 ? 2.2 : 0.7 * q;
+                m /= q;
+            }
+        return held(R) ? c : c + 4.0 * R;
+    }
+    void run(int m, int limit, int depth, double c, int max_last) {
+        if (c >= cost || depth > MIX_MAX_STAGES) return;
+        if (m == 1) {
+            if (max_last > 0 && (depth == 0 || cur[depth - 1] > max_last)) return;
+            cost = c;
+            nbest = depth;
+            std::copy(cur, cur + depth, best);
+            return;
+        }
+        if (depth == MIX_MAX_STAGES) return;
+        for (int R = std::min(m, limit); R >= 2; --R) {
+            if (m % R != 0) continue;
+            if (!held(R)) {
+                bool prime = true;
+                for (int q = 2; q * q <= R; ++q) prime &= R % q != 0;
+                if (!prime) continue;
+            }
+            cur[depth] = R;
+            run(m / R, R, depth + 1, c + radix_cost(R), max_last);
         }
     }
+};
+
+void mix_spans(MixPlan& p) {
+    for (int i = 0, Ns = 1; i < p.nst; Ns *= p.radix[i++]) {
+        p.m[i] = p.n / p.radix[i];
+        p.step[i] = p.n / (Ns * p.radix[i]) * p.tw_stride;
+        p.magic[i] = Ns > 1 ? (unsigned)((4294967296ull + Ns - 1) / Ns) : 0u;
+    }
+}
+
+template <typename T, bool LONG>
+int mix_plan(int n, int tw_stride, int max_last, MixPlan& p) {
+    for (int m = n, q = 2; m > 1; ++q)
+        while (m % q == 0) {
+            if (q > MIX_MAX_PRIME)
+                return fail(FFCM_ERR_UNSUPPORTED, "grid dimension has a prime factor above " +
+                                                      std::to_string(MIX_MAX_PRIME) + " (" + std::to_string(q) + ")");
+            m /= q;
+        }
+    MixSearch any, low;
+    any.held = low.held = mix_has_radix<T, LONG>;
+    any.run(n, MIX_MAX_PRIME, 0, 0.0, 0);
+    if (max_last > 0) low.run(n, MIX_MAX_PRIME, 0, 0.0, max_last);
+    const MixSearch& s = low.nbest > 1 && low.nbest <= any.nbest + 1 ? low : any;
+    p = MixPlan{};
+    p.n = n;
+    p.tw_stride = tw_stride;
+    p.nst = s.nbest;
+    std::copy(s.best, s.best + s.nbest, p.radix);
+    if (n == 1) {   // a line of one value: one empty stage
+        p.nst = 1;
+        p.radix[0] = 1;
+    }
+    mix_spans(p);
     return FFCM_OK;
 }
 
-int pow2_floor(int v) {
-    int p = 1;
-    while (p * 2 <= v) p *= 2;
-    return p;
+// The same radices in reverse order (the inverse transform of the z pass).
+MixPlan mix_reverse(const MixPlan& p) {
+    MixPlan r = p;
+    std::reverse(r.radix, r.radix + r.nst);
+    mix_spans(r);
+    return r;
 }
 
 // ---------------------------------------------------------------------------
@@ -444,9 +502,16 @@ struct Engine final : EngineBase {
     StencilParams<T> sp;
     T h3, inv_mu_M;
     CorrConsts<T> cc;
-    FftPlan plan_x, plan_y, plan_z;
-    int lpb_x, tx_y, tx_z;
-    size_t smem_x, smem_y, smem_z, smem_stencil;
+    // mixed-radix passes (fft_mixed.cuh), per axis: lines per block (1 << lb),
+    // threads and shared memory
+    MixPlan plan_x, plan_y, plan_z, plan_zi;
+    struct MixShape {
+        int lb = 0, threads = 0;
+        bool longl = false;   // the kernels that leave the twiddle table in global memory
+        size_t smem = 0;
+    } mx, my, mz;
+    int z_fuse = 0;
+    size_t smem_stencil;
     // register (power-of-two) FFT path, per axis
     bool fast_x = false, fast_y = false, fast_z = false;
     int lpb_fx = 0, By = 0, Bz = 0;
@@ -602,19 +667,59 @@ struct Engine final : EngineBase {
 
         // FFT plans and launch shapes
         const bool xeven = (Mx % 2) == 0;
-        TRY(make_plan(xeven ? Mx / 2 : Mx, xeven ? 2 : 1, plan_x));
-        TRY(make_plan(My, 1, plan_y));
-        TRY(make_plan(Mz, 1, plan_z));
+        TRY((mix_plan<T, false>(xeven ? Mx / 2 : Mx, xeven ? 2 : 1, 0, plan_x)));
+        TRY((mix_plan<T, false>(My, 1, 0, plan_y)));
+        TRY((mix_plan<T, false>(Mz, 1, mix_fuse_radix<T>(), plan_z)));
         const size_t cs = sizeof(cplx<T>);
         const size_t budget = 200 * 1024;
-        lpb_x = std::max(1, std::min(64, (int)(16384 / (plan_x.n * cs))));
-        smem_x = 2 * (size_t)lpb_x * plan_x.n * cs;
-        tx_y = pow2_floor(std::max(1, std::min(16, (int)(32768 / (My * cs)))));
-        smem_y = 2 * (size_t)tx_y * My * cs;
-        tx_z = pow2_floor(std::max(1, std::min(16, (int)(65536 / (3 * Mz * cs)))));
-        smem_z = 2 * (size_t)3 * tx_z * Mz * cs;
-        if (smem_x > budget || smem_y > budget || smem_z > budget)
+        if (2 * plan_x.n * cs > budget || 2 * My * cs > budget || 2 * 3 * (size_t)Mz * cs > budget)
             return fail(FFCM_ERR_UNSUPPORTED, "grid dimension too large for the shared-memory FFT");
+        // Lines per block: 128 bytes of a spectrum row (whole lines of every
+        // global access, shared-memory rows without bank conflicts; 64 for the
+        // Float32 x rows, whose smaller blocks measured 105 against 120 us at
+        // 240 x 200 x 160), halved while a block would not leave room for a
+        // second one on its SM and while there would be fewer than two blocks
+        // per SM. Not below 64 bytes for the first reason (HBM moves 64-byte
+        // pieces) nor 32 for the second (a sector), unless one block would not
+        // fit at all. Threads: the largest stage's butterflies, in equal rounds
+        // of at most `cap` (the launch bounds).
+        auto shape = [&](char axis, MixPlan& q, int nc, int64_t lines, int64_t planes, MixShape& m) -> int {
+            const int cap = sizeof(T) == 8 ? 256 : 512;
+            int lb = sizeof(T) == 4 && axis != 'x' ? 4 : 3;
+            auto fuses = [&] { return axis == 'z' && q.nst > 1 && q.radix[q.nst - 1] <= mix_fuse_radix<T>(); };
+            auto fit = [&](int l) {
+                const int last = q.nst - 1;
+                int most = 1;
+                for (int i = 0; i < q.nst; ++i) most = std::max(most, nc * (q.m[i] << l));
+                // the z pass: one projector butterfly a thread where that fits
+                const bool mid = fuses() && (q.m[last] << l) <= cap;
+                if (mid) most = q.m[last] << l;
+                const int rounds = (most + cap - 1) / cap;
+                m.lb = l;
+                m.threads = ((most + rounds - 1) / rounds + 31) / 32 * 32;
+                const bool second = axis == 'x' || q.nst > 2 || (axis == 'z' && q.nst == 2 && !mid);
+                const size_t pitch = axis == 'x' && l ? (1 << l) + 1 : 1 << l;
+                m.smem = ((m.longl ? 0 : axis == 'x' ? Mx : q.n) + (second ? 2 : 1) * nc * q.n * pitch) * cs;
+                return m.smem;
+            };
+            while (fit(lb) > 110 * 1024 && (cs << lb) > 64) --lb;
+            while (lb > 0 && fit(lb) > 226 * 1024) --lb;
+            if (fit(lb) > 226 * 1024) {
+                m.longl = true;
+                TRY((mix_plan<T, true>(q.n, q.tw_stride, axis == 'z' ? mix_fuse_radix<T>() : 0, q)));
+            }
+            while (((lines + (1 << lb) - 1) >> lb) * planes < 2 * num_sms && (cs << lb) > 32) --lb;
+            fit(lb);
+            if (axis == 'z') {
+                plan_zi = mix_reverse(q);
+                z_fuse = fuses();
+            }
+            return FFCM_OK;
+        };
+        const int64_t xlines = xeven ? 3 * (int64_t)My * Mz : (3 * (int64_t)My * Mz + 1) / 2;
+        TRY(shape('x', plan_x, 1, xlines, 1, mx));
+        TRY(shape('y', plan_y, 1, nkx, 3 * (int64_t)Mz, my));
+        TRY(shape('z', plan_z, 3, nkx, My, mz));
         smem_stencil = 8 * 3 * (size_t)MG * (2 * sizeof(T) + sizeof(int));
         fast_x = xeven && fast_len(Mx / 2);
         fast_y = fast_len(My);
@@ -696,10 +801,10 @@ struct Engine final : EngineBase {
             if (fast_z && zpipe_kernel<T>(Mz, B) && zpitch % B == 0 && zpipe_smem<T>(Mz, B) <= budget)
                 TRY(raise_smem_cap((const void*)zpipe_kernel<T>(Mz, B), zpipe_smem<T>(Mz, B)));
         }
-        TRY(raise_smem_cap((const void*)k_fft_x_r2c<T>, smem_x));
-        TRY(raise_smem_cap((const void*)k_fft_x_c2r<T>, smem_x));
-        TRY(raise_smem_cap((const void*)k_fft_y<T>, smem_y));
-        TRY(raise_smem_cap((const void*)k_fft_z_stokes<T>, smem_z));
+        TRY(raise_smem_cap((const void*)(mx.longl ? k_fftm_x_r2c<T, true> : k_fftm_x_r2c<T, false>), mx.smem));
+        TRY(raise_smem_cap((const void*)(mx.longl ? k_fftm_x_c2r<T, true> : k_fftm_x_c2r<T, false>), mx.smem));
+        TRY(raise_smem_cap((const void*)(my.longl ? k_fftm_y<T, true> : k_fftm_y<T, false>), my.smem));
+        TRY(raise_smem_cap((const void*)(mz.longl ? k_fftm_z_stokes<T, true> : k_fftm_z_stokes<T, false>), mz.smem));
         if (smem_stencil > 48 * 1024) {
             TRY(raise_smem_cap((const void*)k_spread_atomic<T>, smem_stencil));
             TRY(raise_smem_cap((const void*)k_interpolate_warp<T>, smem_stencil));
@@ -1524,9 +1629,9 @@ struct Engine final : EngineBase {
             return launch(h, y_kernel<T>(My, By), g, By * (My / 8), FastFft<T>::yz_smem(My, By), s, spec,
                           k0, k1, My, mzl, hxp, (const cplx<T>*)twy, inverse);
         }
-        dim3 gy((nkx + tx_y - 1) / tx_y, mzl, 3);
-        return launch(h, k_fft_y<T>, gy, 256, smem_y, s, spec, nkx, My, mzl, hxp, plan_y,
-                      (const cplx<T>*)twy, tx_y, inverse);
+        dim3 gy((nkx + (1 << my.lb) - 1) >> my.lb, mzl, 3);
+        return launch(h, my.longl ? k_fftm_y<T, true> : k_fftm_y<T, false>, gy, my.threads, my.smem, s, spec, hxp, plan_y, (const cplx<T>*)twy, my.lb,
+                      inverse);
     }
 
     int launch_z(cudaStream_t s, int k0 = 0, int k1 = 0) {
@@ -1562,9 +1667,9 @@ struct Engine final : EngineBase {
                           k0, k1, My, zpitch, (const cplx<T>*)twz, kxz, (const T*)kyv,
                           (const T*)kzv, inv_mu_M);
         }
-        dim3 gz((nkz + tx_z - 1) / tx_z, My, 1);
-        return launch(h, k_fft_z_stokes<T>, gz, 256, smem_z, s, zbuf, nkz, My, Mz, zpitch, plan_z,
-                      (const cplx<T>*)twz, tx_z, kxz, (const T*)kyv, (const T*)kzv, inv_mu_M);
+        dim3 gz((nkz + (1 << mz.lb) - 1) >> mz.lb, My, 1);
+        return launch(h, mz.longl ? k_fftm_z_stokes<T, true> : k_fftm_z_stokes<T, false>, gz, mz.threads, mz.smem, s, zbuf, nkz, My, zpitch, plan_z, plan_zi,
+                      z_fuse, (const cplx<T>*)twz, mz.lb, kxz, (const T*)kyv, (const T*)kzv, inv_mu_M);
     }
 
     int stokes(cudaStream_t s) override {
@@ -1579,8 +1684,9 @@ struct Engine final : EngineBase {
             return launch(h, xf_kernel<T>(H), (nrows + lpb_fx - 1) / lpb_fx, lpb_fx * (H / 8), smem_fx, s, in,
                           spec, nrows, hxp, (const cplx<T>*)twx, lpb_fx);
         }
-        return launch(h, k_fft_x_r2c<T>, (nrows + lpb_x - 1) / lpb_x, 256, smem_x, s, in, spec, Mx, nrows, hxp,
-                      plan_x, (const cplx<T>*)twx, lpb_x);
+        const int nlines = Mx % 2 == 0 ? nrows : (nrows + 1) / 2;
+        return launch(h, mx.longl ? k_fftm_x_r2c<T, true> : k_fftm_x_r2c<T, false>, (nlines + (1 << mx.lb) - 1) >> mx.lb, mx.threads, mx.smem, s, in, spec, Mx,
+                      nrows, hxp, plan_x, (const cplx<T>*)twx, mx.lb);
     }
 
     int x_inverse(T* out, cudaStream_t s) {
@@ -1590,8 +1696,9 @@ struct Engine final : EngineBase {
             return launch(h, xi_kernel<T>(H), (nrows + lpb_fx - 1) / lpb_fx, lpb_fx * (H / 8), smem_fx, s,
                           (const cplx<T>*)spec, out, nrows, hxp, (const cplx<T>*)twx, lpb_fx);
         }
-        return launch(h, k_fft_x_c2r<T>, (nrows + lpb_x - 1) / lpb_x, 256, smem_x, s, (const cplx<T>*)spec, out,
-                      Mx, nrows, hxp, plan_x, (const cplx<T>*)twx, lpb_x);
+        const int nlines = Mx % 2 == 0 ? nrows : (nrows + 1) / 2;
+        return launch(h, mx.longl ? k_fftm_x_c2r<T, true> : k_fftm_x_c2r<T, false>, (nlines + (1 << mx.lb) - 1) >> mx.lb, mx.threads, mx.smem, s,
+                      (const cplx<T>*)spec, out, Mx, nrows, hxp, plan_x, (const cplx<T>*)twx, mx.lb);
     }
 
     // gf -> out through the full transform and the Stokes projector.

@@ -10,7 +10,7 @@
 // same positions, so the passes below load and store HBM directly, coalesced.
 // Twiddles W_n^t come from a shared-memory copy of the per-axis table.
 //
-// Same five passes and conventions as fft.cuh (x r2c, y, z + projector, y
+// Same five passes and conventions as fft_mixed.cuh (x r2c, y, z + projector, y
 // inverse, x c2r; c2r ignores the imaginary parts of the x DC and Nyquist
 // bins).
 #pragma once
@@ -27,7 +27,7 @@ __host__ __device__ constexpr int padded_len(int n) { return n + n / 8 + 1; }
 
 template <typename T>
 __device__ __forceinline__ void dft8(cplx<T> (&v)[8], bool inv) {
-    SmallDft<T, 8>::run(v, inv, nullptr, 0);
+    SmallDft<T, 8>::run(v, inv);
 }
 
 template <typename T>
@@ -159,7 +159,7 @@ __device__ __forceinline__ void dft_small(cplx<T> (&a)[L], bool inv) {
     if constexpr (L == 4) {
         dft4(a[0], a[1], a[2], a[3], inv);
     } else if constexpr (L == 8) {
-        SmallDft<T, 8>::run(a, inv, nullptr, 0);
+        SmallDft<T, 8>::run(a, inv);
     } else {
         static_assert(L == 16, "L must be 4, 8 or 16");
         dft16(a, inv);
