@@ -29,6 +29,42 @@ template <typename T>
 __device__ __forceinline__ cplx<T> csub(cplx<T> a, cplx<T> b) { return {a.x - b.x, a.y - b.y}; }
 template <typename T>
 __device__ __forceinline__ cplx<T> cconj(cplx<T> a) { return {a.x, -a.y}; }
+
+// Two neighbouring values of T whose sums and products are one instruction in
+// Float32 (f32x2, each half rounded as its scalar form).
+template <typename T>
+struct pair2;
+template <>
+struct pair2<float> {
+    unsigned long long v;
+    __device__ __forceinline__ pair2() {}
+    __device__ __forceinline__ pair2(float x, float y) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y)); }
+    __device__ __forceinline__ float x() const { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return a; }
+    __device__ __forceinline__ float y() const { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return b; }
+};
+template <>
+struct pair2<double> {
+    double a, b;
+    __device__ __forceinline__ pair2() {}
+    __device__ __forceinline__ pair2(double x, double y) : a(x), b(y) {}
+    __device__ __forceinline__ double x() const { return a; }
+    __device__ __forceinline__ double y() const { return b; }
+};
+__device__ __forceinline__ pair2<float> mul2(pair2<float> a, pair2<float> b) {
+    pair2<float> r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ pair2<float> fma2(pair2<float> a, pair2<float> b, pair2<float> c) {
+    pair2<float> r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ pair2<double> mul2(pair2<double> a, pair2<double> b) { return {a.a * b.a, a.b * b.b}; }
+__device__ __forceinline__ pair2<double> fma2(pair2<double> a, pair2<double> b, pair2<double> c) {
+    return {__fma_rn(a.a, b.a, c.a), __fma_rn(a.b, b.b, c.b)};
+}
+
 // multiply by -i (forward) or +i (inverse)
 template <typename T>
 __device__ __forceinline__ cplx<T> mul_mi(cplx<T> a) { return {a.y, -a.x}; }

@@ -27,6 +27,7 @@
 #include "fft_mixed.cuh"
 #include "fft_pipe.cuh"
 #include "fft_tma.cuh"
+#include "pencil.cuh"
 #include "slab.cuh"
 #include "spread_interp.cuh"
 
@@ -325,6 +326,9 @@ struct EngineBase {
     virtual void* adj_buf(int which) = 0;  // 0 lambda, 1 dY, 2 dF, 3 target, 4 J (double)
     virtual int ensure_real_grids() = 0;
     virtual bool uses_slab() const = 0;
+    // the assembled solve works from particle lists that depend on the
+    // positions only (ensure_lists)
+    virtual bool keeps_lists() const = 0;
     // stencil arithmetic of every later launch (FFCM_STENCIL_*)
     virtual void set_stencil(int mode) = 0;
     // the y/z variant in use: ykind, By, ygrid, zkind, Bz, zgrid, kx_chunk
@@ -554,6 +558,13 @@ struct Engine final : EngineBase {
     int* slab_lists = nullptr;   // per-slab particle lists kept by the spread
     int* slab_counts = nullptr;
     int ntiles;
+    // pencil kernels: spread and interpolation on the real grid where the slab
+    // kernels do not apply; CSR lists over (pencil, first x point)
+    bool pencil = false;
+    PencilKernels<T> pk;
+    PencilGeom pg;
+    int pen_bins = 0;
+    int *pen_cnt = nullptr, *pen_off = nullptr, *pen_ent = nullptr, *pen_used = nullptr;
 
     T *Yin = nullptr, *Fin = nullptr, *Vout = nullptr, *Yw = nullptr;
     int32_t *key = nullptr, *perm = nullptr, *cnt = nullptr, *off = nullptr, *tiles = nullptr;
@@ -697,6 +708,10 @@ struct Engine final : EngineBase {
                 const int rounds = (most + cap - 1) / cap;
                 m.lb = l;
                 m.threads = ((most + rounds - 1) / rounds + 31) / 32 * 32;
+                // x rows are loaded and stored a warp each: three warps at least
+                // (240 x 200 x 160: 105 us a pass with 96 threads, 155 with 256,
+                // whose registers leave an SM two blocks)
+                if (axis == 'x') m.threads = std::max(m.threads, 96);
                 const bool second = axis == 'x' || q.nst > 2 || (axis == 'z' && q.nst == 2 && !mid);
                 const size_t pitch = axis == 'x' && l ? (1 << l) + 1 : 1 << l;
                 m.smem = ((m.longl ? 0 : axis == 'x' ? Mx : q.n) + (second ? 2 : 1) * nc * q.n * pitch) * cs;
@@ -754,6 +769,20 @@ struct Engine final : EngineBase {
             sg.lcap = (sg.lcap + 31) / 32 * 32;
             TRY(raise_smem_cap((const void*)sk.spread_fused, sk.smem));
             TRY(raise_smem_cap((const void*)sk.interp, sk.smem_interp));
+        }
+        pg.nty = (My + PENCIL_TY - 1) / PENCIL_TY;
+        pg.ntz = (Mz + PENCIL_TZ - 1) / PENCIL_TZ;
+        if (!slab && !h->distributed && (int64_t)pg.nty * pg.ntz * Mx < (1 << 30) && pencil_pays() &&
+            pencil_kernels<T>(MG, pk)) {
+            pencil = true;
+            pen_bins = pg.nty * pg.ntz * Mx;
+            // segments: about 24 warps per SM, each of at least four stencils
+            const int npen = pg.nty * pg.ntz, piece = 32 / (int)sizeof(T);
+            const int want = std::max(1, std::min((num_sms * 24 + npen - 1) / npen, Mx / (4 * MG)));
+            pg.seg = ((Mx + want - 1) / want + piece - 1) / piece * piece;
+            pg.nseg = (Mx + pg.seg - 1) / pg.seg;
+            TRY(raise_smem_cap((const void*)pk.spread, pk.smem));
+            TRY(raise_smem_cap((const void*)pk.interp, pk.smem_interp));
         }
         mzl = Mz;
         zpitch = hxp;
@@ -846,6 +875,16 @@ struct Engine final : EngineBase {
             TRY(alloc(partial, 3 * (size_t)N));
             TRY(alloc(slab_lists, (size_t)sg.nty * sg.ntz * sg.lcap));
             TRY(alloc(slab_counts, (size_t)sg.nty * sg.ntz));
+        }
+
+        if (pencil) {
+            TRY(alloc(partial, 3 * (size_t)N));
+            TRY(alloc(pen_cnt, pen_bins));
+            TRY(alloc(pen_off, (size_t)pen_bins + (size_t)pg.nty * pg.ntz));
+            TRY(alloc(pen_used, 1));
+            TRY(alloc(pen_ent, (size_t)N * pencil_reach(PENCIL_TY, MG, My) * pencil_reach(PENCIL_TZ, MG, Mz)));
+            CUDA_TRY(cudaMemset(pen_cnt, 0, (size_t)pen_bins * sizeof(int)));
+            CUDA_TRY(cudaMemset(pen_used, 0, sizeof(int)));
         }
 
         // zero-initialised grids and cell list (src/config.jl:443-448)
@@ -1171,6 +1210,7 @@ struct Engine final : EngineBase {
     }
 
     bool uses_slab() const override { return slab; }
+    bool keeps_lists() const override { return slab || pencil; }
     void set_stencil(int mode) override { sp.comp = mode == FFCM_STENCIL_FLOAT64 ? 1 : 0; }
 
     int gather_forces(const void* F, cudaStream_t s) override {
@@ -1205,6 +1245,47 @@ struct Engine final : EngineBase {
         return launch(h, k_rank_gather<T>, grid_for(N, 256), 256, 0, s, N, (const int32_t*)key,
                       (const int32_t*)off, (const int32_t*)scratch_i, perm, (const T*)Yw,
                       static_cast<const T*>(F), Ys, Fs);
+    }
+
+    // Whether the pencil kernels beat one warp per particle (global atomics in
+    // the spread). Their cost grows with the pencils a particle reaches and, as
+    // every pencil is walked whether or not it holds particles, with the grid;
+    // the lists are three more launches. Spread + interpolation, warp per
+    // particle against pencils, by stencil points N M_G^3 and their ratio to the
+    // grid's points: 187M, 11: 1458 / 687 us (Float64 1822 / 1191); 86M, 2.6:
+    // 695 / 557; 43M, 1.3 (Float64): 838 / 876; 15M, 7: 130 / 137; 15M, 1.9:
+    // 144 / 193. FFCM_PENCIL = 0 or 1 forces the choice.
+    bool pencil_pays() const {
+        if (const char* v = std::getenv("FFCM_PENCIL")) return v[0] == '1';
+        const double points = (double)N * MG * MG * MG;
+        return points >= 2e7 && points >= 2.5 * (double)plane;
+    }
+
+    // The pencils' particle lists of the sorted positions.
+    int pencil_lists(cudaStream_t s) {
+        StageScope sc(h, FFCM_STAGE_SPREAD, s);
+        const int npen = pg.nty * pg.ntz;
+        TRY(launch(h, k_pencil_count<T>, grid_for((int64_t)N * PENCIL_SPLIT, 128), 128, 0, s, N, (const vec4<T>*)Ys, sp, pg, pen_cnt));
+        TRY(launch(h, k_pencil_offsets, (npen + 7) / 8, 256, 0, s, npen, Mx, (const int*)pen_cnt, pen_off, pen_used));
+        return launch(h, k_pencil_scatter<T>, grid_for((int64_t)N * PENCIL_SPLIT, 128), 128, 0, s, N, (const vec4<T>*)Ys, sp, pg,
+                      (const int*)pen_off, pen_cnt, pen_ent, pen_used);
+    }
+
+    int pencil_blocks() const { return (pg.nty * pg.ntz * pg.nseg + PENCIL_WARPS - 1) / PENCIL_WARPS; }
+
+    // forces -> force density on the real grid (every point written)
+    int pencil_spread(const vec4<T>* force, cudaStream_t s) {
+        StageScope sc(h, FFCM_STAGE_SPREAD, s);
+        return launch(h, pk.spread, pencil_blocks(), 32 * PENCIL_WARPS, pk.smem, s, (const vec4<T>*)Ys, force, sp, pg,
+                      (const int*)pen_off, (const int*)pen_ent, gf);
+    }
+
+    // velocities gu -> h^-3 V in sorted order in `partial`
+    int pencil_interp(cudaStream_t s) {
+        StageScope sc(h, FFCM_STAGE_INTERPOLATE, s);
+        CUDA_TRY(cudaMemsetAsync(partial, 0, 3 * (size_t)N * sizeof(T), s));
+        return launch(h, pk.interp, pencil_blocks(), 32 * PENCIL_WARPS, pk.smem_interp, s, (const vec4<T>*)Ys, sp, pg,
+                      (const int*)pen_off, (const int*)pen_ent, (const T*)gu, partial);
     }
 
     // Hot path of the assembled operator: spread straight into the x-transformed
@@ -1283,6 +1364,7 @@ struct Engine final : EngineBase {
                        slab_lists, slab_counts));
         } else {
             TRY(ensure_real_grids());
+            if (pencil) TRY(pencil_lists(s));
         }
         lists_built = true;
         return FFCM_OK;
@@ -1310,21 +1392,31 @@ struct Engine final : EngineBase {
     // keep_u: also leave the velocity grid u = L^-1 S F in gu (the adjoint's
     // only checkpoint); the unfused pipeline leaves it there anyway.
     int solve(void* V, cudaStream_t s, bool keep_u, bool build_lists = true) {
-        if (!slab) {
+        if (!slab && !pencil) {
             TRY(spread(s));
             TRY(stokes(s));
             TRY(interp(V, s));
             return correct(V, s);
         }
-        TRY(spread_to_spectrum(s, nullptr, build_lists));
+        if (slab) {
+            TRY(spread_to_spectrum(s, nullptr, build_lists));
+        } else {
+            TRY(ensure_real_grids());
+            if (build_lists) TRY(pencil_lists(s));
+            TRY(pencil_spread(Fs, s));
+        }
         bool side = false, probe = false;
         TRY(fork_pairs(s, side, probe));
+        if (pencil) {
+            StageScope sc(h, FFCM_STAGE_FFT_X_FWD, s);
+            TRY(x_forward(gf, s));
+        }
         TRY(stokes_yz(s, probe ? h->ev_probe : nullptr));
-        if (keep_u) {
+        if (keep_u || pencil) {
             StageScope sc(h, FFCM_STAGE_FFT_X_INV, s);
             TRY(x_inverse(gu, s));
         }
-        TRY(interp_from_spectrum(s));
+        TRY(pencil ? pencil_interp(s) : interp_from_spectrum(s));
         if (side) {
             // (the correction stage's time is the side stream's pair kernel's)
             CUDA_TRY(cudaStreamWaitEvent(s, h->ev_join, 0));
@@ -1583,7 +1675,7 @@ struct Engine final : EngineBase {
             StageScope sc(h, FFCM_STAGE_FFT_X_INV, s);
             TRY(x_inverse(gpsi, s));
         } else {
-            TRY(spread_from(Ls, s));
+            TRY(pencil ? pencil_spread(Ls, s) : spread_from(Ls, s));   // the checkpoint's lists
             TRY(stokes_to(gpsi, s));
         }
         {
@@ -2254,7 +2346,7 @@ int ffcm_mobility(ffcm_handle* h, void* V, int64_t vr, int64_t vc, const void* Y
     const void* Yd = Y;
     const void* Fd = F;
     void* Vd = V;
-    if (memory == FFCM_HOST && e->uses_slab()) {
+    if (memory == FFCM_HOST && e->keeps_lists()) {
         // The positions go first; the forces follow on the copy stream
         // (after the positions' copy and so after the work queued on s before
         // it, which may still read the staging buffer) while the positions

@@ -1,0 +1,99 @@
+"""Pencil spread and interpolation (csrc/pencil.cuh), forced on with FFCM_PENCIL=1,
+against the oracle: grids whose sides are no multiple of a pencil or of a
+segment, stencils of every instance width and as wide as the grid, particles
+on one spot, at the box edges and alone; and the paths that keep the lists
+(operator, conjugate gradients, adjoint, batch capture)."""
+import numpy as np
+import pytest
+
+from gpu_helpers import both, kw_of, rel_l2
+
+import ffcm_oracle as O
+
+pytestmark = pytest.mark.gpu
+# the end-to-end parity bounds of the whole suite (test_gpu_mobility.py)
+TOL = {np.float32: 1e-5, np.float64: 1e-10}
+
+
+def _inputs(T, L, N, layout, seed):
+    rng = np.random.default_rng(seed)
+    L = np.broadcast_to(np.asarray(L, np.float64), (3,))
+    Y = rng.random((N, 3)) * L
+    if layout == "spot":          # more than one batch of entries with one first x point
+        Y = 0.3 * L + 0.05 * rng.standard_normal((N, 3))
+    elif layout == "edges":       # half of them within a tenth of the box of a face, no two alike
+        Y[::2] = np.mod(0.2 * (Y[::2] - 0.5 * L), L)
+    return Y.astype(T), rng.standard_normal((N, 3)).astype(T)
+
+
+@pytest.fixture
+def forced(monkeypatch):
+    monkeypatch.setenv("FFCM_PENCIL", "1")
+    return monkeypatch
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+@pytest.mark.parametrize("M,MG,N,layout", [
+    ((10, 12, 14), 6, 40, "uniform"), ((10, 12, 14), 10, 40, "edges"), ((7, 9, 8), 7, 30, "uniform"),
+    ((33, 17, 9), 9, 300, "edges"), ((24, 8, 4), 4, 60, "uniform"), ((12, 12, 12), 12, 50, "edges"),
+    ((40, 30, 50), 7, 900, "uniform"), ((100, 31, 29), 11, 700, "edges"), ((96, 40, 36), 12, 500, "uniform"),
+    ((130, 24, 20), 5, 400, "edges"), ((64, 64, 64), 10, 1500, "uniform"), ((45, 33, 30), 8, 200, "spot"),
+    ((20, 18, 22), 2, 100, "uniform"), ((60, 60, 60), 9, 1, "uniform"),
+])
+def test_pencil_solve_matches_oracle(ffcm, forced, T, M, MG, N, layout):
+    L = tuple(0.6 * m for m in M)
+    prod, ora = both(ffcm, T, **kw_of(L, N, M, M_G=MG, R_c=0.4 * min(L)))
+    Y, F = _inputs(T, L, N, layout, N + MG)
+    V = np.empty_like(Y)
+    for _ in range(2):            # the second solve reuses the list buffers
+        ffcm.mobility(V, prod, Y, F)
+    if layout == "spot":
+        # the pair terms of overlapping spheres cancel badly in Float32, in the
+        # oracle as here: compare with the same pair terms beside the
+        # warp-per-particle grid steps
+        forced.setenv("FFCM_PENCIL", "0")
+        ref = ffcm.mobility(np.empty_like(Y), ffcm.FFCMConfig(T, **kw_of(L, N, M, M_G=MG, R_c=0.4 * min(L))), Y, F)
+    else:
+        ref = O.apply(ora, Y, F)
+    assert rel_l2(V, ref) < TOL[T]
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+def test_pencil_lists_are_kept(ffcm, forced, T):
+    """Operator, conjugate gradients and adjoint on kept lists: the same as
+    without the pencils, in either stencil mode."""
+    M, N, L = (50, 36, 42), 600, tuple(0.55 * m for m in (50, 36, 42))
+    kw = kw_of(L, N, M, M_G=9, R_c=3.0)
+    Y, F = _inputs(T, L, N, "uniform", 3)
+    lam = F[::-1].copy()
+    got = []
+    for mode in "10":
+        forced.setenv("FFCM_PENCIL", mode)
+        cfg = ffcm.FFCMConfig(T, **kw)
+        res = []
+        for stencil in ("reference", "float64"):
+            cfg.stencil = stencil
+            A = ffcm.FFCMMobility(cfg, Y)
+            res += [A @ F, A @ lam, ffcm.cg(A, F, reltol=0.0, maxiter=5)]
+            V, pull = ffcm.rrule_mobility(cfg, Y, F)
+            res += [V, *pull(lam)]
+        got.append(res)
+    for a, b in zip(*got):
+        assert rel_l2(a, b) < 10 * TOL[T]   # five iterations and the gradient's cancellation
+
+
+def test_pencil_batch_under_capture(ffcm, forced):
+    T = np.float32
+    systems = [dict(L=(27.0,) * 3, R_c=3.0, N=400, num_grid_points=(48, 48, 48)),
+               dict(L=(30.0, 15.0, 20.0), R_c=3.0, N=200, num_grid_points=(60, 30, 40))]
+    b = ffcm.FFCMBatch(T, systems=systems, kernel_widths_ratio=2.0, M_G=9, viscosity=1.0, nrhs=2)
+    rng = np.random.default_rng(0)
+    Ys = [(rng.random((s["N"], 3)) * np.array(s["L"])).astype(T) for s in systems]
+    Fs = [[rng.standard_normal((s["N"], 3)).astype(T) for _ in range(2)] for s in systems]
+    Yp, Fp = b.pack(Ys, Fs)
+    V = np.empty_like(Fp)
+    b.mobility(V, Yp, Fp)
+    for s, Y, fs, vs in zip(systems, Ys, Fs, b.unpack(V)):
+        ora = O.OracleConfig(T, kernel_widths_ratio=2.0, M_G=9, viscosity=1.0, **s)
+        for f, v in zip(fs, vs):
+            assert rel_l2(v, O.apply(ora, Y, f)) < TOL[T]
