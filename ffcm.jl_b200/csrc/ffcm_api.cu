@@ -1444,7 +1444,10 @@ struct Engine final : EngineBase {
     // FFCM_OVERLAP_PAIRS forces a mode, the first solve runs on one stream
     // with events around its y forward pass and its correction, and a later
     // solve, once those have completed, fixes the mode for the configuration:
-    // overlap when the correction took under half the y pass. `side` tells
+    // overlap when the correction took under half the y pass and the y pass over
+    // 0.4 ms (a short y pass ends before the correction, whose blocks then delay
+    // the z pass's single wave: 256^3 Float64, N = 62,500: 1641 us on one
+    // stream, 1690 us overlapped; Float32 732 / 736). `side` tells
     // the caller whether it forked, `probe` whether to record the events
     // (ev_probe[0..1] around the y forward pass, [2..3] around k_correct).
     // Under capture (the batched graph, the CG loop) the solve keeps the
@@ -1479,7 +1482,7 @@ struct Engine final : EngineBase {
                 float ty = 0, tc = 0;
                 CUDA_TRY(cudaEventElapsedTime(&ty, h->ev_probe[0], h->ev_probe[1]));
                 CUDA_TRY(cudaEventElapsedTime(&tc, h->ev_probe[2], h->ev_probe[3]));
-                h->pair_overlap = tc < 0.5f * ty;
+                h->pair_overlap = tc < 0.5f * ty && ty > 0.4f;
                 h->pair_probe = 2;
             }
             if (!h->pair_overlap) return FFCM_OK;
