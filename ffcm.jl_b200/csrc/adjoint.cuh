@@ -170,7 +170,7 @@ __global__ void k_correct_adjoint(int n_part, const vec4<T>* __restrict__ Ys, co
                                   CorrConsts<T> c, CorrGradConsts<T> cg) {
     // TPP lanes per particle share its 27 neighbour cells (as in k_correct)
     const int sub = threadIdx.x % TPP;
-    const unsigned group = ((1u << TPP) - 1u) << (lane_id() & ~(TPP - 1));
+    const unsigned group = corr_group<TPP>();
     const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)n_part * TPP;
          t += nthreads) {

@@ -39,8 +39,8 @@ struct pair2<float> {
     unsigned long long v;
     __device__ __forceinline__ pair2() {}
     __device__ __forceinline__ pair2(float x, float y) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y)); }
-    __device__ __forceinline__ float x() const { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return a; }
-    __device__ __forceinline__ float y() const { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return b; }
+    __device__ __forceinline__ float x() const { return __uint_as_float((unsigned)v); }
+    __device__ __forceinline__ float y() const { return __uint_as_float((unsigned)(v >> 32)); }
 };
 template <>
 struct pair2<double> {

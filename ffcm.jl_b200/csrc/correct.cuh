@@ -66,7 +66,16 @@ __device__ __forceinline__ T min_image(T x, T L) {
 // Vs == nullptr: V[:, perm[s]] += dv (the step API, reference semantics).
 // Vs != nullptr: V[:, perm[s]] = h3 * Vs[s] + dv (finishes the fused
 // interpolation, which left its sums in sorted order in Vs).
-inline int corr_tpp(int64_t n_part) { return n_part <= 200000 ? 4 : 1; }
+inline int corr_tpp(int64_t n_part) {
+    return n_part <= 16000 ? 32 : n_part <= 50000 ? 8 : n_part <= 200000 ? 4 : 1;
+}
+
+// Lanes of the TPP-lane group a lane belongs to.
+template <int TPP>
+__device__ __forceinline__ unsigned corr_group() {
+    if (TPP == 32) return 0xffffffffu;
+    return ((1u << (TPP % 32)) - 1u) << (lane_id() & ~(TPP - 1));
+}
 
 // Self term plus the pair terms of sorted particle s over its 27 neighbour
 // cells; lane `sub` of the particle's TPP-lane group takes cells q = sub,
@@ -138,7 +147,7 @@ __global__ void k_correct(int n_part, const vec4<T>* __restrict__ Ys,
                           const int32_t* __restrict__ perm, T* __restrict__ V, CorrConsts<T> c,
                           const T* __restrict__ Vs, T h3) {
     const int sub = threadIdx.x % TPP;
-    const unsigned group = ((1u << TPP) - 1u) << (lane_id() & ~(TPP - 1));
+    const unsigned group = corr_group<TPP>();
     const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)n_part * TPP;
          t += nthreads) {
@@ -168,7 +177,7 @@ template <typename T, int TPP>
 __global__ void k_correct_pairs(int n_part, const vec4<T>* __restrict__ Ys, const vec4<T>* __restrict__ Fs,
                                 const int32_t* __restrict__ off, CorrConsts<T> c, T* __restrict__ dv) {
     const int sub = threadIdx.x % TPP;
-    const unsigned group = ((1u << TPP) - 1u) << (lane_id() & ~(TPP - 1));
+    const unsigned group = corr_group<TPP>();
     const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)n_part * TPP;
          t += nthreads) {

@@ -303,8 +303,14 @@ std::map<TuneKey, TunedChoice>& tune_store() {
 
 struct EngineBase {
     virtual ~EngineBase() = default;
-    virtual int wrap_hash(const void* Y, bool wrap, bool hash, cudaStream_t s) = 0;
-    virtual int sort(const void* F, cudaStream_t s) = 0;
+    virtual int wrap_hash(const void* Y, bool wrap, bool hash, cudaStream_t s, bool count = false) = 0;
+    // counted: the cells were counted by the wrap_hash before
+    virtual int sort(const void* F, cudaStream_t s, bool counted = false) = 0;
+    // wrap, hash and sort: the cell list of positions Y
+    int cell_list(const void* Y, const void* F, cudaStream_t s) {
+        const int rc = wrap_hash(Y, true, true, s, true);
+        return rc != FFCM_OK ? rc : sort(F, s, true);
+    }
     virtual int spread(cudaStream_t s) = 0;
     virtual int stokes(cudaStream_t s) = 0;
     virtual int interp(void* V, cudaStream_t s) = 0;
@@ -492,6 +498,9 @@ __global__ void k_copy_block(cplx<T>* __restrict__ dst, int64_t dc, int64_t dz, 
         for (int k = threadIdx.x; k < nk; k += blockDim.x) d[k] = s[k];
     }
 }
+
+// The instance of a correction kernel for N particles.
+#define FFCM_CORR(K) (corr_tpp(N) == 32 ? K<T, 32> : corr_tpp(N) == 8 ? K<T, 8> : corr_tpp(N) == 4 ? K<T, 4> : K<T, 1>)
 
 template <typename T>
 struct Engine final : EngineBase {
@@ -891,6 +900,7 @@ struct Engine final : EngineBase {
         CUDA_TRY(cudaMemset(spec, 0, 3 * (size_t)hxp * My * mzl * sizeof(cplx<T>)));
         if (fast_z || fast_y) make_tma_maps();
         CUDA_TRY(cudaMemset(off, 0, ((size_t)ncell + 1) * sizeof(int32_t)));
+        CUDA_TRY(cudaMemset(cnt, 0, (size_t)ncell * sizeof(int32_t)));   // zero between cell lists
         CUDA_TRY(cudaMemset(perm, 0, (size_t)N * sizeof(int32_t)));
         CUDA_TRY(cudaMemset(key, 0, (size_t)N * sizeof(int32_t)));
         CUDA_TRY(cudaMemset(Yw, 0, 3 * (size_t)N * sizeof(T)));
@@ -1223,23 +1233,25 @@ struct Engine final : EngineBase {
     void* F_in() override { return Fin; }
     void* V_out() override { return Vout; }
 
-    int wrap_hash(const void* Y, bool wrap, bool hash, cudaStream_t s) override {
+    int wrap_hash(const void* Y, bool wrap, bool hash, cudaStream_t s, bool count) override {
         StageScope sc(h, FFCM_STAGE_CELL_LIST, s);
         return launch(h, k_wrap_hash<T>, grid_for(N, 256), 256, 0, s, N,
                       static_cast<const T*>(Y), Yw, key, L[0], L[1], L[2], d.inv_cell_size[0],
                       d.inv_cell_size[1], d.inv_cell_size[2], m0, m1, m2, h->d_err,
-                      wrap ? 1 : 0, hash ? 1 : 0);
+                      wrap ? 1 : 0, hash ? 1 : 0, count ? cnt : nullptr);
     }
 
-    int sort(const void* F, cudaStream_t s) override {
+    int sort(const void* F, cudaStream_t s, bool counted) override {
         StageScope sc(h, FFCM_STAGE_CELL_LIST, s);
-        CUDA_TRY(cudaMemsetAsync(cnt, 0, (size_t)ncell * sizeof(int32_t), s));
-        TRY(launch(h, k_count_cells, grid_for(N, 256), 256, 0, s, N, (const int32_t*)key, cnt));
-        TRY(launch(h, k_scan_tiles, ntiles, SCAN_THREADS, 0, s, (const int32_t*)cnt, ncell, tiles));
-        TRY(launch(h, k_scan_tile_sums, 1, 1024, 0, s, tiles, ntiles));
-        TRY(launch(h, k_scan_apply, ntiles, SCAN_THREADS, 0, s, (const int32_t*)cnt, ncell,
-                   (const int32_t*)tiles, off));
-        CUDA_TRY(cudaMemsetAsync(cnt, 0, (size_t)ncell * sizeof(int32_t), s));
+        if (!counted) TRY(launch(h, k_count_cells, grid_for(N, 256), 256, 0, s, N, (const int32_t*)key, cnt));
+        if (ncell <= SCAN_ONE_PASS) {
+            TRY(launch(h, k_scan_one_pass, ntiles, SCAN_THREADS, 0, s, (const int32_t*)cnt, ncell, off));
+        } else {
+            TRY(launch(h, k_scan_tiles, ntiles, SCAN_THREADS, 0, s, (const int32_t*)cnt, ncell, tiles));
+            TRY(launch(h, k_scan_tile_sums, 1, 1024, 0, s, tiles, ntiles));
+            TRY(launch(h, k_scan_apply, ntiles, SCAN_THREADS, 0, s, (const int32_t*)cnt, ncell,
+                       (const int32_t*)tiles, off));
+        }
         TRY(launch(h, k_scatter_cells, grid_for(N, 256), 256, 0, s, N, (const int32_t*)key,
                    (const int32_t*)off, cnt, scratch_i));
         return launch(h, k_rank_gather<T>, grid_for(N, 256), 256, 0, s, N, (const int32_t*)key,
@@ -1253,12 +1265,13 @@ struct Engine final : EngineBase {
     // the lists are three more launches. Spread + interpolation, warp per
     // particle against pencils, by stencil points N M_G^3 and their ratio to the
     // grid's points: 187M, 11: 1458 / 687 us (Float64 1822 / 1191); 86M, 2.6:
-    // 695 / 557; 43M, 1.3 (Float64): 838 / 876; 15M, 7: 130 / 137; 15M, 1.9:
-    // 144 / 193. FFCM_PENCIL = 0 or 1 forces the choice.
+    // 695 / 557; 43M, 1.3 (Float64): 838 / 876; 23M, 3.3: 191 / 192 (Float64
+    // 274 / 314, whose pencils keep fewer warps on an SM); 15M, 7: 130 / 137;
+    // 15M, 1.9: 144 / 193. FFCM_PENCIL = 0 or 1 forces the choice.
     bool pencil_pays() const {
         if (const char* v = std::getenv("FFCM_PENCIL")) return v[0] == '1';
         const double points = (double)N * MG * MG * MG;
-        return points >= 2e7 && points >= 2.5 * (double)plane;
+        return points >= (sizeof(T) == 4 ? 2e7 : 5e7) && points >= 2.5 * (double)plane;
     }
 
     // The pencils' particle lists of the sorted positions.
@@ -1273,17 +1286,17 @@ struct Engine final : EngineBase {
 
     int pencil_blocks() const { return (pg.nty * pg.ntz * pg.nseg + PENCIL_WARPS - 1) / PENCIL_WARPS; }
 
-    // forces -> force density on the real grid (every point written)
+    // forces -> force density on the real grid (every point written); `partial`
+    // zeroed for the interpolation
     int pencil_spread(const vec4<T>* force, cudaStream_t s) {
         StageScope sc(h, FFCM_STAGE_SPREAD, s);
         return launch(h, pk.spread, pencil_blocks(), 32 * PENCIL_WARPS, pk.smem, s, (const vec4<T>*)Ys, force, sp, pg,
-                      (const int*)pen_off, (const int*)pen_ent, gf);
+                      (const int*)pen_off, (const int*)pen_ent, gf, partial, 3 * (int64_t)N);
     }
 
     // velocities gu -> h^-3 V in sorted order in `partial`
     int pencil_interp(cudaStream_t s) {
         StageScope sc(h, FFCM_STAGE_INTERPOLATE, s);
-        CUDA_TRY(cudaMemsetAsync(partial, 0, 3 * (size_t)N * sizeof(T), s));
         return launch(h, pk.interp, pencil_blocks(), 32 * PENCIL_WARPS, pk.smem_interp, s, (const vec4<T>*)Ys, sp, pg,
                       (const int*)pen_off, (const int*)pen_ent, (const T*)gu, partial);
     }
@@ -1302,7 +1315,7 @@ struct Engine final : EngineBase {
         return launch(h, sk.spread_fused, g, 256, sk.smem, s, (const vec4<T>*)Ys,
                       force ? force : (const vec4<T>*)Fs,
                       (const int32_t*)off, spec, hxp, sp, sg, (const cplx<T>*)twx, (const int*)slab_lists,
-                      (const int*)slab_counts);
+                      (const int*)slab_counts, partial, 3 * (int64_t)N);
     }
 
     // y forward, z + projector, y inverse. With kx chunking (kx_chunk > 0) the
@@ -1339,7 +1352,6 @@ struct Engine final : EngineBase {
     // x-c2r + gather; leaves h^-3 V in sorted order in `partial` for correct_final.
     int interp_from_spectrum(cudaStream_t s) {
         StageScope sc(h, FFCM_STAGE_INTERPOLATE, s);
-        CUDA_TRY(cudaMemsetAsync(partial, 0, 3 * (size_t)N * sizeof(T), s));
         dim3 g(sg.nty, sg.ntz, 1);
         return launch(h, sk.interp, g, 256, sk.smem_interp, s, (const vec4<T>*)Ys, (const int32_t*)off,
                       (const cplx<T>*)spec, hxp, partial, sp, sg, (const cplx<T>*)twx,
@@ -1425,7 +1437,7 @@ struct Engine final : EngineBase {
         }
         StageScope sc(h, FFCM_STAGE_CORRECT, s);
         if (probe) CUDA_TRY(cudaEventRecord(h->ev_probe[2], s));
-        TRY(launch(h, corr_tpp(N) == 4 ? k_correct<T, 4> : k_correct<T, 1>, grid_for((int64_t)N * corr_tpp(N), 128), 128, 0, s, N, (const vec4<T>*)Ys,
+        TRY(launch(h, FFCM_CORR(k_correct), grid_for((int64_t)N * corr_tpp(N), 128), 128, 0, s, N, (const vec4<T>*)Ys,
                    (const vec4<T>*)Fs, (const int32_t*)off, (const int32_t*)perm,
                    static_cast<T*>(V), cc, (const T*)partial, h3));
         if (probe) CUDA_TRY(cudaEventRecord(h->ev_probe[3], s));
@@ -1497,7 +1509,7 @@ struct Engine final : EngineBase {
         CUDA_TRY(cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0));
         {
             StageScope sc(h, FFCM_STAGE_CORRECT, h->side_stream);
-            TRY(launch(h, corr_tpp(N) == 4 ? k_correct_pairs<T, 4> : k_correct_pairs<T, 1>,
+            TRY(launch(h, FFCM_CORR(k_correct_pairs),
                        grid_for((int64_t)N * corr_tpp(N), 128), 128, 0, h->side_stream, N, (const vec4<T>*)Ys,
                        (const vec4<T>*)Fs, (const int32_t*)off, cc, dvs));
         }
@@ -1554,8 +1566,7 @@ struct Engine final : EngineBase {
     // planes, y forward; then the first transpose's send blocks: peer q gets
     // this rank's planes at q's kx columns.
     int dist_forward(const void* Y, const void* F, cudaStream_t s) override {
-        TRY(wrap_hash(Y, true, true, s));
-        TRY(sort(F, s));
+        TRY(cell_list(Y, F, s));
         TRY(spread_to_spectrum(s, nullptr, true));
         {
             StageScope sc(h, FFCM_STAGE_FFT_Y_FWD, s);
@@ -1601,7 +1612,7 @@ struct Engine final : EngineBase {
     // V = h^3 partial + the pair correction, with `partial` summed over ranks.
     int dist_correct(void* V, cudaStream_t s) override {
         StageScope sc(h, FFCM_STAGE_CORRECT, s);
-        return launch(h, corr_tpp(N) == 4 ? k_correct<T, 4> : k_correct<T, 1>, grid_for((int64_t)N * corr_tpp(N), 128),
+        return launch(h, FFCM_CORR(k_correct), grid_for((int64_t)N * corr_tpp(N), 128),
                       128, 0, s, N, (const vec4<T>*)Ys, (const vec4<T>*)Fs, (const int32_t*)off, (const int32_t*)perm,
                       static_cast<T*>(V), cc, (const T*)partial, h3);
     }
@@ -1688,7 +1699,7 @@ struct Engine final : EngineBase {
                        (const T*)gu, (const T*)gpsi, static_cast<T*>(dY), static_cast<T*>(dF), sp, h3));
         }
         StageScope sc(h, FFCM_STAGE_CORRECT, s);
-        return launch(h, corr_tpp(N) == 4 ? k_correct_adjoint<T, 4> : k_correct_adjoint<T, 1>,
+        return launch(h, FFCM_CORR(k_correct_adjoint),
                       grid_for((int64_t)N * corr_tpp(N), 128), 128, 0, s, N, (const vec4<T>*)Ys,
                       (const vec4<T>*)Fs, (const vec4<T>*)Ls, (const int32_t*)off, (const int32_t*)perm,
                       static_cast<T*>(dY), static_cast<T*>(dF), cc, cgc);
@@ -1817,7 +1828,7 @@ struct Engine final : EngineBase {
 
     int correct(void* V, cudaStream_t s) override {
         StageScope sc(h, FFCM_STAGE_CORRECT, s);
-        return launch(h, corr_tpp(N) == 4 ? k_correct<T, 4> : k_correct<T, 1>, grid_for((int64_t)N * corr_tpp(N), 128), 128, 0, s, N, (const vec4<T>*)Ys,
+        return launch(h, FFCM_CORR(k_correct), grid_for((int64_t)N * corr_tpp(N), 128), 128, 0, s, N, (const vec4<T>*)Ys,
                       (const vec4<T>*)Fs, (const int32_t*)off, (const int32_t*)perm,
                       static_cast<T*>(V), cc, (const T*)nullptr, T(0));
     }
@@ -2370,8 +2381,7 @@ int ffcm_mobility(ffcm_handle* h, void* V, int64_t vr, int64_t vc, const void* Y
             CUDA_TRY(cudaMemcpyAsync(e->F_in(), F, bytes, cudaMemcpyHostToDevice, h->copy_stream));
             CUDA_TRY(cudaEventRecord(h->ev_forces, h->copy_stream));
         }
-        TRY(e->wrap_hash(e->Y_in(), true, true, s));
-        TRY(e->sort(nullptr, s));
+        TRY(e->cell_list(e->Y_in(), nullptr, s));
         e->lists_built = false;
         TRY(e->ensure_lists(s));
         CUDA_TRY(cudaStreamWaitEvent(s, h->ev_forces, 0));
@@ -2391,8 +2401,7 @@ int ffcm_mobility(ffcm_handle* h, void* V, int64_t vr, int64_t vc, const void* Y
         Fd = e->F_in();
         Vd = e->V_out();
     }
-    TRY(e->wrap_hash(Yd, true, true, s));
-    TRY(e->sort(Fd, s));
+    TRY(e->cell_list(Yd, Fd, s));
     TRY(e->mobility_rest(Vd, s));
     if (memory == FFCM_HOST) {
         {
@@ -2522,8 +2531,7 @@ int ffcm_mobility_checkpoint(ffcm_handle* h, void* V, const void* Y, const void*
         Fd = e->F_in();
         Vd = e->V_out();
     }
-    TRY(e->wrap_hash(Yd, true, true, s));
-    TRY(e->sort(Fd, s));
+    TRY(e->cell_list(Yd, Fd, s));
     TRY(e->forward_checkpoint(Vd, s));
     h->ckpt = true;
     if (memory == FFCM_HOST) {
@@ -2594,8 +2602,7 @@ int ffcm_objective_gradient(ffcm_handle* h, double* J, void* dJdY, void* dJdF, v
         dYd = e->adj_buf(1);
         dFd = e->adj_buf(2);
     }
-    TRY(e->wrap_hash(Yd, true, true, s));
-    TRY(e->sort(Fd, s));
+    TRY(e->cell_list(Yd, Fd, s));
     TRY(e->forward_checkpoint(Vd, s));
     TRY(e->residual(Vd, Td, e->adj_buf(0), Jdev, s));
     TRY(e->adjoint(e->adj_buf(0), dYd, dFd, s));
@@ -2635,8 +2642,7 @@ int ffcm_set_positions(ffcm_handle* h, const void* Y, int32_t memory, void* stre
     }
     // the sort gathers some forces along; zeros stand in until the first apply
     CUDA_TRY(cudaMemsetAsync(e->F_in(), 0, bytes, s));
-    TRY(e->wrap_hash(Yd, true, true, s));
-    TRY(e->sort(e->F_in(), s));
+    TRY(e->cell_list(Yd, e->F_in(), s));
     e->lists_built = false;
     if (memory == FFCM_HOST) TRY(finish(h, s));
     h->positions = true;
@@ -2981,8 +2987,7 @@ int batch_build_graph(ffcm_batch* b) {
         const char* Y = static_cast<const char*>(b->Yb) + 3 * b->yoff[i] * es;
         auto Fr = [&](int r) { return static_cast<const char*>(b->Fb) + (b->fvoff[i] + 3 * r * b->N[i]) * es; };
         auto Vr = [&](int r) { return static_cast<char*>(b->Vb) + (b->fvoff[i] + 3 * r * b->N[i]) * es; };
-        rc = e->wrap_hash(Y, true, true, s);
-        if (rc == FFCM_OK) rc = e->sort(Fr(0), s);
+        rc = e->cell_list(Y, Fr(0), s);
         if (rc == FFCM_OK) rc = e->mobility_rest(Vr(0), s);
         for (int r = 1; r < b->nrhs && rc == FFCM_OK; ++r) {
             rc = e->gather_forces(Fr(r), s);

@@ -310,9 +310,12 @@ __device__ __forceinline__ void mix_run_stage(const MixPlan& p, int s, int Ns, i
 // `sm`, where the block starts copying it, or from global memory (LONG).
 template <typename T, bool LONG>
 __device__ __forceinline__ const cplx<T>* mix_table(cplx<T>* sm, const cplx<T>* __restrict__ table, int count) {
-    if constexpr (LONG) return table;
-    for (int i = threadIdx.x; i < count; i += blockDim.x) sm[i] = table[i];
-    return sm;
+    if constexpr (LONG) {
+        return table;
+    } else {
+        for (int i = threadIdx.x; i < count; i += blockDim.x) sm[i] = table[i];
+        return sm;
+    }
 }
 
 // ---- y c2c on (kx tile) x My columns of one (c, z) plane ------------------

@@ -251,12 +251,13 @@ template <typename T, int MGT>
 __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 10 : 6)
     k_pencil_spread(const vec4<T>* __restrict__ Ys, const vec4<T>* __restrict__ Fs, const __grid_constant__
                     StencilParams<T> p, PencilGeom g, const int* __restrict__ off, const int* __restrict__ ent,
-                    T* __restrict__ grid) {
+                    T* __restrict__ grid, T* __restrict__ Vs, int64_t nvs) {
     using Warp = PencilWarp<T, MGT>;
     constexpr int XC = Warp::XC;
-    extern __shared__ __align__(32) unsigned char smem_raw[];
+    zero_sums(Vs, nvs);
+    extern __shared__ __align__(32) unsigned char pencil_smem[];
     const int lane = threadIdx.x & 31;
-    PencilSpreadWarp<T, MGT>& S = reinterpret_cast<PencilSpreadWarp<T, MGT>*>(smem_raw)[threadIdx.x >> 5];
+    PencilSpreadWarp<T, MGT>& S = reinterpret_cast<PencilSpreadWarp<T, MGT>*>(pencil_smem)[threadIdx.x >> 5];
     Warp& W = S.w;
     const int task = blockIdx.x * PENCIL_WARPS + (threadIdx.x >> 5);
     if (task >= g.nty * g.ntz * g.nseg) return;   // whole warps
@@ -364,9 +365,9 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 8 : 5)
                     T* __restrict__ Vs) {
     using Warp = PencilWarp<T, MGT>;
     constexpr int XC = Warp::XC;
-    extern __shared__ __align__(32) unsigned char smem_raw[];
+    extern __shared__ __align__(32) unsigned char pencil_smem[];
     const int lane = threadIdx.x & 31;
-    PencilInterpWarp<T, MGT>& I = reinterpret_cast<PencilInterpWarp<T, MGT>*>(smem_raw)[threadIdx.x >> 5];
+    PencilInterpWarp<T, MGT>& I = reinterpret_cast<PencilInterpWarp<T, MGT>*>(pencil_smem)[threadIdx.x >> 5];
     Warp& W = I.w;
     constexpr int SUM_GROUP = PencilInterpWarp<T, MGT>::SUM_GROUP;
     const int task = blockIdx.x * PENCIL_WARPS + (threadIdx.x >> 5);
@@ -471,7 +472,7 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 8 : 5)
 
 template <typename T>
 using PencilSpreadKernel = void (*)(const vec4<T>*, const vec4<T>*, const StencilParams<T>, PencilGeom, const int*,
-                                    const int*, T*);
+                                    const int*, T*, T*, int64_t);
 template <typename T>
 using PencilInterpKernel = void (*)(const vec4<T>*, const StencilParams<T>, PencilGeom, const int*, const int*,
                                     const T*, T*);

@@ -209,13 +209,31 @@ __global__ void k_slab_lists(const vec4<T>* __restrict__ Ys, const int32_t* __re
     int* out = lists + (int64_t)slab * g.lcap;
     const unsigned lt = (1u << lane) - 1u;
     int total = 0;
-    for (int pi = 0; pi < rows.ny * rows.nz; ++pi) {
-        const int c0 = slab_row_cell(g, rows, pi);
-        const int sb = off[c0], se = off[c0 + g.m0];
-        for (int b = sb; b < se; b += 32) {
-            const int s = b + lane;
+    // up to 32 cell rows at a time, one per lane; the candidates of all of them
+    // in row order, 32 at a time
+    for (int p0 = 0; p0 < rows.ny * rows.nz; p0 += 32) {
+        int sb = 0, n = 0;
+        if (p0 + lane < rows.ny * rows.nz) {
+            const int c0 = slab_row_cell(g, rows, p0 + lane);
+            sb = off[c0];
+            n = off[c0 + g.m0] - sb;
+        }
+        int end = n;   // candidates up to and including the lane's row
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, end, d);
+            if (lane >= d) end += t;
+        }
+        const int all = __shfl_sync(0xffffffffu, end, 31);
+        for (int b = 0; b < all; b += 32) {
+            // the row of candidate b + lane: the first whose end exceeds it
+            int r = 0;
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1)
+                if (__shfl_sync(0xffffffffu, end, r + d - 1) <= b + lane) r += d;
+            const int s = b + lane - __shfl_sync(0xffffffffu, end - n, r) + __shfl_sync(0xffffffffu, sb, r);
             unsigned m = 0;
-            if (s < se) {
+            if (b + lane < all) {
                 int sx, sy, sz;
                 slab_anchor<T, BY, BZ>(p, Ys[s], y0r, z0r, sx, sy, sz, m);
             }
@@ -392,6 +410,14 @@ __device__ __forceinline__ void slab_x_r2c(T* acc, cplx<T>* __restrict__ spec, i
     }
 }
 
+// The interpolation's sums, zeroed by the spread of the same solve (the blocks
+// of a one-dimensional or two-dimensional grid share them evenly).
+template <typename T>
+__device__ __forceinline__ void zero_sums(T* __restrict__ Vs, int64_t n) {
+    const int64_t block = blockIdx.x + (int64_t)blockIdx.y * gridDim.x, step = (int64_t)gridDim.x * gridDim.y * blockDim.x;
+    for (int64_t i = block * blockDim.x + threadIdx.x; i < n; i += step) Vs[i] = T(0);
+}
+
 // ---- spread into a slab, then x-r2c straight into the spectrum -----------
 template <typename T, int H, int BY, int BZ>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_spread_slab(const vec4<T>* __restrict__ Ys,
@@ -401,8 +427,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_spread_slab(con
                                                      StencilParams<T> p, SlabGeom g,
                                                      const cplx<T>* __restrict__ twx,
                                                      const int* __restrict__ lists,
-                                                     const int* __restrict__ counts) {
+                                                     const int* __restrict__ counts, T* __restrict__ Vs,
+                                                     int64_t nvs) {
     constexpr int Mx = 2 * H, P = slab_pitch(Mx), NRP = BY * BZ, ROWS = 3 * NRP;
+    zero_sums(Vs, nvs);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* acc = reinterpret_cast<T*>(smem_raw);
     SpreadWin<T, BY, BZ, H>& W = *reinterpret_cast<SpreadWin<T, BY, BZ, H>*>(acc + ROWS * P);
@@ -773,7 +801,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_interp_slab(con
 // ---- host-side dispatch over the x length ----------------------------------
 template <typename T>
 using SpreadSlabKernel = void (*)(const vec4<T>*, const vec4<T>*, const int32_t*, cplx<T>*, int,
-                                  StencilParams<T>, SlabGeom, const cplx<T>*, const int*, const int*);
+                                  StencilParams<T>, SlabGeom, const cplx<T>*, const int*, const int*, T*, int64_t);
 template <typename T>
 using ListsKernel = void (*)(const vec4<T>*, const int32_t*, StencilParams<T>, SlabGeom, int*, int*);
 template <typename T>
