@@ -65,6 +65,16 @@ struct SlabShape {
     static constexpr int BZ = (2 * H >= 1024) ? 1 : 2;
 };
 
+// Blocks of the slab kernels per SM, which the compiler fits the registers to.
+// They wait on shared memory and on the windows' barriers more than they issue,
+// so a further block per SM is worth some spilled registers wherever shared
+// memory holds it. 256^3, N = 60,000: Float32, 3 to 4 blocks: spread 203 to 183
+// us, interpolation 172 to 155; Float64, 2 to 3: 568 to 457, 470 to 385; and
+// the 512 slabs of a 64^3 grid run at once (spread 17 to 12 us). From x length
+// 512 on shared memory decides.
+template <typename T, int H>
+constexpr int slab_blocks() { return sizeof(T) == 8 ? (H <= 128 ? 3 : 2) : H <= 128 ? 4 : 3; }
+
 // Range of cell indices (along one axis) that can hold a particle whose
 // stencil anchor lies in [lo_anchor, hi_anchor] (unwrapped). The 1e-3 h slack
 // covers the Float32 rounding of y / h and of the cell assignment.
@@ -420,7 +430,7 @@ __device__ __forceinline__ void zero_sums(T* __restrict__ Vs, int64_t n) {
 
 // ---- spread into a slab, then x-r2c straight into the spectrum -----------
 template <typename T, int H, int BY, int BZ>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_spread_slab(const vec4<T>* __restrict__ Ys,
+__global__ void __launch_bounds__(256, slab_blocks<T, H>()) k_spread_slab(const vec4<T>* __restrict__ Ys,
                                                      const vec4<T>* __restrict__ Fs,
                                                      const int32_t* __restrict__ off,
                                                      cplx<T>* __restrict__ spec, int hxp,
@@ -620,7 +630,7 @@ __host__ __device__ constexpr unsigned slab_row_copy_bytes() {
 }
 
 template <typename T, int H, int BY, int BZ>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_interp_slab(const vec4<T>* __restrict__ Ys,
+__global__ void __launch_bounds__(256, slab_blocks<T, H>()) k_interp_slab(const vec4<T>* __restrict__ Ys,
                                                      const int32_t* __restrict__ off,
                                                      const cplx<T>* __restrict__ spec, int hxp,
                                                      T* __restrict__ Vs, StencilParams<T> p,
