@@ -68,12 +68,14 @@ struct SlabShape {
 // Blocks of the slab kernels per SM, which the compiler fits the registers to.
 // They wait on shared memory and on the windows' barriers more than they issue,
 // so a further block per SM is worth some spilled registers wherever shared
-// memory holds it. 256^3, N = 60,000: Float32, 3 to 4 blocks: spread 203 to 183
-// us, interpolation 172 to 155; Float64, 2 to 3: 568 to 457, 470 to 385; and
-// the 512 slabs of a 64^3 grid run at once (spread 17 to 12 us). From x length
-// 512 on shared memory decides.
+// memory holds it. 256^3, N = 60,000, us by blocks: Float32 spread 203 (3), 183
+// (4), 204 (5), interpolation 172 (3), 155 (4), 147 (5), 156 (6); Float64 spread 568 (2),
+// 457 (3), 413 (4), interpolation 470 (2), 385 (3), 374 (4); and the 512 slabs
+// of a 64^3 grid run at once. From x length 512 on shared memory decides.
 template <typename T, int H>
-constexpr int slab_blocks() { return sizeof(T) == 8 ? (H <= 128 ? 3 : 2) : H <= 128 ? 4 : 3; }
+constexpr int spread_blocks() { return H <= 128 ? 4 : sizeof(T) == 8 ? 2 : 3; }
+template <typename T, int H>
+constexpr int interp_blocks() { return H <= 128 ? (sizeof(T) == 8 ? 4 : 5) : sizeof(T) == 8 ? 2 : 3; }
 
 // Range of cell indices (along one axis) that can hold a particle whose
 // stencil anchor lies in [lo_anchor, hi_anchor] (unwrapped). The 1e-3 h slack
@@ -430,7 +432,7 @@ __device__ __forceinline__ void zero_sums(T* __restrict__ Vs, int64_t n) {
 
 // ---- spread into a slab, then x-r2c straight into the spectrum -----------
 template <typename T, int H, int BY, int BZ>
-__global__ void __launch_bounds__(256, slab_blocks<T, H>()) k_spread_slab(const vec4<T>* __restrict__ Ys,
+__global__ void __launch_bounds__(256, spread_blocks<T, H>()) k_spread_slab(const vec4<T>* __restrict__ Ys,
                                                      const vec4<T>* __restrict__ Fs,
                                                      const int32_t* __restrict__ off,
                                                      cplx<T>* __restrict__ spec, int hxp,
@@ -630,7 +632,7 @@ __host__ __device__ constexpr unsigned slab_row_copy_bytes() {
 }
 
 template <typename T, int H, int BY, int BZ>
-__global__ void __launch_bounds__(256, slab_blocks<T, H>()) k_interp_slab(const vec4<T>* __restrict__ Ys,
+__global__ void __launch_bounds__(256, interp_blocks<T, H>()) k_interp_slab(const vec4<T>* __restrict__ Ys,
                                                      const int32_t* __restrict__ off,
                                                      const cplx<T>* __restrict__ spec, int hxp,
                                                      T* __restrict__ Vs, StencilParams<T> p,
