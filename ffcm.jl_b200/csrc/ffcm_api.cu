@@ -697,7 +697,7 @@ struct Engine final : EngineBase {
         // Lines per block: 128 bytes of a spectrum row (whole lines of every
         // global access, shared-memory rows without bank conflicts; 64 for the
         // Float32 x rows, whose smaller blocks measured 105 against 120 us at
-        // 240 x 200 x 160), halved while a block would not leave room for a
+        // 240 x 200 x 160 before their loads were asynchronous), halved while a block would not leave room for a
         // second one on its SM and while there would be fewer than two blocks
         // per SM. Not below 64 bytes for the first reason (HBM moves 64-byte
         // pieces) nor 32 for the second (a sector), unless one block would not

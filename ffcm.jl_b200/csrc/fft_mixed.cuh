@@ -33,7 +33,9 @@
 // issue slots, shared-memory conflicts negligible, DRAM at 1.5-2 TB/s).
 // Measured there, against runtime-radix stages of radix 2, 4, 8 and odd primes
 // with every stage through shared memory: y 312 -> 58 us, z and projector
-// 818 -> 84 us, x r2c 155 -> 104 us, x c2r 140 -> 113 us (93 MB spectrum).
+// 818 -> 84 us, x r2c 155 -> 79 us, x c2r 140 -> 86 us (93 MB spectrum; the x
+// passes at 104 and 113 us with their rows loaded through registers, which left
+// too few loads in flight).
 #pragma once
 
 #include "common.cuh"
@@ -503,6 +505,16 @@ __device__ __forceinline__ const cplx<T>* mix_lines(const MixPlan& p, MixBuf<T> 
     return cur.p;
 }
 
+// B bytes (4, 8, 16; both addresses aligned to them) from global to shared
+// memory without passing through registers.
+template <int B>
+__device__ __forceinline__ void copy_async(void* shared, const void* global) {
+    const unsigned to = (unsigned)__cvta_generic_to_shared(shared);
+    if constexpr (B == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(global) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(to), "l"(global), "n"(B) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ---- x r2c, rows of the real grid -> rows of the spectrum -----------------
 // Even Mx: the row's Mx/2 pairs as one complex line of length Mx/2 (twiddle
 // stride 2). Odd Mx: two rows as the real and imaginary part of one line of
@@ -521,17 +533,24 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256)
     const int per = even ? 1 : 2, nlines = (nrows + per - 1) / per;
     const int line0 = blockIdx.x << lb, nl = min(1 << lb, nlines - line0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    // all of the block's rows in flight at once
     for (int b = warp; b < nl; b += nw) {
         const int64_t row = (int64_t)(line0 + b) * per;
         if (even) {
             const cplx<T>* src = reinterpret_cast<const cplx<T>*>(f + row * Mx);
-            for (int i = lane; i < n; i += 32) A[i * pitch + b] = src[i];
+            for (int i = lane; i < n; i += 32) copy_async<sizeof(cplx<T>)>(A + i * pitch + b, src + i);
         } else {
+            const T* src = f + row * Mx;
             const bool two = row + 1 < nrows;
-            for (int i = lane; i < n; i += 32)
-                A[i * pitch + b] = cplx<T>{f[row * Mx + i], two ? f[(row + 1) * Mx + i] : T(0)};
+            for (int i = lane; i < n; i += 32) {
+                cplx<T>* to = A + i * pitch + b;
+                copy_async<sizeof(T)>(&to->x, src + i);
+                if (two) copy_async<sizeof(T)>(&to->y, src + Mx + i);
+                else to->y = T(0);
+            }
         }
     }
+    copy_async_wait();
     __syncthreads();
     const cplx<T>* Z = mix_lines<T, LONG>(p, MixBuf<T>{A, pitch, 0}, MixBuf<T>{A + n * pitch, pitch, 0}, lb, tw);
     const int nk = Mx / 2 + 1;
@@ -569,31 +588,43 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256)
     const int per = even ? 1 : 2, nlines = (nrows + per - 1) / per;
     const int line0 = blockIdx.x << lb, nl = min(1 << lb, nlines - line0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int b = warp; b < nl; b += nw) {
-        const int64_t row = (int64_t)(line0 + b) * per;
-        const cplx<T>* src = spec + row * hxp;
-        const bool two = !even && row + 1 < nrows;
-        for (int k = lane; k < n; k += 32) {
-            cplx<T> z;
-            if (even) {
-                cplx<T> Xk = src[k], Xc = src[n - k];
+    // bins k and n - k of a row make the line's values k and n - k
+    if (even) {
+        // all of the block's rows in flight at once (bin n lies in the second
+        // buffer, which the stages use later)
+        for (int b = warp; b < nl; b += nw) {
+            const cplx<T>* src = spec + (int64_t)(line0 + b) * hxp;
+            for (int k = lane; k <= n; k += 32) copy_async<sizeof(cplx<T>)>(A + k * pitch + b, src + k);
+        }
+        copy_async_wait();
+        __syncthreads();
+        for (int b = warp; b < nl; b += nw) {
+            for (int k = lane; 2 * k <= n; k += 32) {
+                cplx<T> Xk = A[k * pitch + b], Xc = A[(n - k) * pitch + b];
                 if (k == 0) {
                     Xk.y = T(0);  // DC imaginary part ignored
                     Xc.y = T(0);  // Nyquist imaginary part ignored
                 }
-                const cplx<T> S = cadd(Xk, cconj(Xc));
-                z = cadd(S, mul_pi(cmul(csub(Xk, cconj(Xc)), cconj(table[k]))));
-            } else {
-                const int q = 2 * k <= n ? k : n - k;
-                cplx<T> Xa = src[q], Xb = two ? src[hxp + q] : cplx<T>{T(0), T(0)};
-                if (q == 0) Xa.y = Xb.y = T(0);
-                if (q != k) {
-                    Xa.y = -Xa.y;
-                    Xb.y = -Xb.y;
-                }
-                z = cadd(Xa, mul_pi(Xb));
+                const cplx<T> S = cadd(Xk, cconj(Xc)), D = csub(Xk, cconj(Xc));
+                A[k * pitch + b] = cadd(S, mul_pi(cmul(D, cconj(tw[k]))));
+                // value n - k: the conjugate sum, and minus the conjugate difference
+                if (k > 0)
+                    A[(n - k) * pitch + b] =
+                        csub(cconj(S), mul_pi(cmul(cconj(D), cconj(tw[n - k]))));
             }
-            A[k * pitch + b] = z;
+        }
+    } else {
+        for (int b = warp; b < nl; b += nw) {
+            const int64_t row = (int64_t)(line0 + b) * per;
+            const cplx<T>* src = spec + row * hxp;
+            const bool two = row + 1 < nrows;
+#pragma unroll 4
+            for (int k = lane; 2 * k < n; k += 32) {
+                cplx<T> Xa = src[k], Xb = two ? src[hxp + k] : cplx<T>{T(0), T(0)};
+                if (k == 0) Xa.y = Xb.y = T(0);
+                A[k * pitch + b] = cadd(Xa, mul_pi(Xb));
+                if (k > 0) A[(n - k) * pitch + b] = cadd(cconj(Xa), mul_pi(cconj(Xb)));
+            }
         }
     }
     __syncthreads();
