@@ -781,8 +781,10 @@ struct Engine final : EngineBase {
         }
         pg.nty = (My + PENCIL_TY - 1) / PENCIL_TY;
         pg.ntz = (Mz + PENCIL_TZ - 1) / PENCIL_TZ;
-        if (!slab && !h->distributed && (int64_t)pg.nty * pg.ntz * Mx < (1 << 30) && pencil_pays() &&
-            pencil_kernels<T>(MG, pk)) {
+        // (bins and list entries are counted in 32 bits)
+        if (!slab && !h->distributed && (int64_t)pg.nty * pg.ntz * Mx < (1 << 30) &&
+            (int64_t)N * pencil_reach(PENCIL_TY, MG, My) * pencil_reach(PENCIL_TZ, MG, Mz) < (1ll << 31) &&
+            pencil_pays() && pencil_kernels<T>(MG, pk)) {
             pencil = true;
             pen_bins = pg.nty * pg.ntz * Mx;
             // segments: about 24 warps per SM, each of at least four stencils
@@ -1606,6 +1608,9 @@ struct Engine final : EngineBase {
                                dist.recv + q * dist.blk, bc(), bz(), dist.nk_max, mzl, My, dist.ke[q] - dist.kb[q], s));
             TRY(launch_y(s, 1));
         }
+        // (the spread zeroed the sums of the first call; a call repeated on the
+        // same received blocks starts from zero too)
+        CUDA_TRY(cudaMemsetAsync(partial, 0, 3 * (size_t)N * sizeof(T), s));
         return interp_from_spectrum(s);
     }
 
@@ -2315,8 +2320,10 @@ int ffcm_set_stencil(ffcm_handle* h, int32_t mode) {
     h->stencil = mode;
     h->eng->set_stencil(mode);
     // a checkpoint was made with the other weights, and the conjugate-gradient
-    // graph holds the old kernel parameters: neither may be reused
+    // graph holds the old kernel parameters: neither may be reused; the particle
+    // lists of fixed positions are in the old mode's anchors
     h->ckpt = false;
+    h->eng->lists_built = false;
     cg_release(h);
     return FFCM_OK;
 }

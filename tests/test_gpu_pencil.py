@@ -82,6 +82,29 @@ def test_pencil_lists_are_kept(ffcm, forced, T):
         assert rel_l2(a, b) < 10 * TOL[T]   # five iterations and the gradient's cancellation
 
 
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+def test_stencil_switch_on_fixed_positions(ffcm, forced, T):
+    """The lists follow a stencil mode changed after the positions were fixed
+    (positions half way between grid points, whose anchors depend on the mode)."""
+    M, N = (50, 36, 42), 400
+    L = tuple(0.537 * m for m in M)
+    cfg = ffcm.FFCMConfig(T, **kw_of(L, N, M, M_G=9, R_c=3.0))
+    rng = np.random.default_rng(8)
+    Y = ((rng.integers(0, np.array(M), (N, 3)) + 0.5) * np.array(L) / np.array(M)
+         + 1e-9 * rng.standard_normal((N, 3))).astype(T)
+    Y = Y[np.unique(Y, axis=0, return_index=True)[1]]
+    Y = np.concatenate([Y, (rng.random((N - len(Y), 3)) * np.array(L)).astype(T)])
+    F = rng.standard_normal((N, 3)).astype(T)
+    A = ffcm.FFCMMobility(cfg, Y)
+    A @ F
+    for mode in ("float64", "reference"):
+        cfg.stencil = mode
+        got = A @ F
+        assert rel_l2(got, ffcm.mobility(np.empty_like(F), cfg, Y, F)) < TOL[T]
+        A = ffcm.FFCMMobility(cfg, Y)
+        A @ F
+
+
 def test_pencil_batch_under_capture(ffcm, forced):
     T = np.float32
     systems = [dict(L=(27.0,) * 3, R_c=3.0, N=400, num_grid_points=(48, 48, 48)),
