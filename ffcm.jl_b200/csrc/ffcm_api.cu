@@ -890,12 +890,14 @@ struct Engine final : EngineBase {
 
         if (pencil) {
             TRY(alloc(partial, 3 * (size_t)N));
-            TRY(alloc(pen_cnt, pen_bins));
-            TRY(alloc(pen_off, (size_t)pen_bins + (size_t)pg.nty * pg.ntz));
-            TRY(alloc(pen_used, 1));
-            TRY(alloc(pen_ent, (size_t)N * pencil_reach(PENCIL_TY, MG, My) * pencil_reach(PENCIL_TZ, MG, Mz)));
-            CUDA_TRY(cudaMemset(pen_cnt, 0, (size_t)pen_bins * sizeof(int)));
-            CUDA_TRY(cudaMemset(pen_used, 0, sizeof(int)));
+            // one allocation (each costs 0.2 to 0.3 ms): counts, entries used, offsets, entries
+            const size_t noff = (size_t)pen_bins + (size_t)pg.nty * pg.ntz;
+            const size_t nent = (size_t)N * pencil_reach(PENCIL_TY, MG, My) * pencil_reach(PENCIL_TZ, MG, Mz);
+            TRY(alloc(pen_cnt, (size_t)pen_bins + 1 + noff + nent));
+            pen_used = pen_cnt + pen_bins;
+            pen_off = pen_used + 1;
+            pen_ent = pen_off + noff;
+            CUDA_TRY(cudaMemset(pen_cnt, 0, ((size_t)pen_bins + 1) * sizeof(int)));
         }
 
         // zero-initialised grids and cell list (src/config.jl:443-448)

@@ -30,7 +30,7 @@
 //
 // What bounds it: the issue of the butterflies' and address instructions at the
 // few warps their registers leave (ncu at 240 x 200 x 160, Float32: 40-48% of
-// issue slots, shared-memory conflicts negligible, DRAM at 1.5-2 TB/s).
+// issue slots, shared-memory conflicts negligible, DRAM at 0.8-1.6 TB/s).
 // Measured there, against runtime-radix stages of radix 2, 4, 8 and odd primes
 // with every stage through shared memory: y 312 -> 58 us, z and projector
 // 818 -> 84 us, x r2c 155 -> 79 us, x c2r 140 -> 86 us (93 MB spectrum; the x
