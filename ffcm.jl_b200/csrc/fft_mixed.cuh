@@ -53,7 +53,7 @@ constexpr int MIX_MAX_STAGES = 14;
 template <typename T, bool LONG>
 __host__ __device__ constexpr bool mix_has_radix(int R) {
     if (LONG) return R == 2 || R == 3 || R == 4 || R == 5 || R == 7 || R == 8;
-    return R <= 16 || (sizeof(T) == 4 && (R == 18 || R == 20 || R == 25));
+    return (R >= 2 && R <= 16) || (sizeof(T) == 4 && (R == 18 || R == 20 || R == 25));
 }
 constexpr int MIX_MAX_PRIME = 61;    // largest prime factor of a line length
 
@@ -320,6 +320,14 @@ __device__ __forceinline__ const cplx<T>* mix_table(cplx<T>* sm, const cplx<T>* 
     }
 }
 
+// Before a first stage that reads global memory: the prime stage, alone among
+// them, takes twiddles in its first stage too, so it waits for the copy of the
+// table (the others wait at the barrier after the stage).
+template <typename T, bool LONG>
+__device__ __forceinline__ void mix_first_wait(const MixPlan& p) {
+    if (!LONG && !mix_has_radix<T, LONG>(p.radix[0])) __syncthreads();
+}
+
 // ---- y c2c on (kx tile) x My columns of one (c, z) plane ------------------
 template <typename T, bool LONG>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256)
@@ -333,6 +341,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256)
     // whole tiles: the row pitch is a multiple of the tile width, the padding
     // columns hold whatever they held, transformed
     const MixSpan<T> g{spec + ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * n * hxp + (blockIdx.x << lb), hxp, 0};
+    mix_first_wait<T, LONG>(p);
     mix_run_stage<T, LONG, 1, MIX_FIRST>(p, 0, 1, lb, tw, g, cur);
     __syncthreads();
     int Ns = p.radix[0];
@@ -443,6 +452,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256, sizeof(T) == 4 ? 1
         cur = other;
         other = t;
     };
+    mix_first_wait<T, LONG>(p);
     mix_run_stage<T, LONG, 3, MIX_FIRST>(p, 0, 1, lb, tw, g, cur);
     __syncthreads();
     // forward up to the stage the projector is fused with, then the inverse

@@ -38,3 +38,25 @@ def test_stokes_solve_of_any_grid(ffcm, T, M):
     ffcm.stokes_solve(prod)
     O.stokes_solve(ora)
     assert rel_l2(prod.fluid_velocity, ora.fluid_velocity) < UNITS * np.finfo(T).eps
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+@pytest.mark.parametrize("M", [(64, 136, 32), (64, 32, 136), (48, 24, 228), (96, 204, 30), (96, 30, 114)])
+def test_prime_first_stage_of_many_warps(ffcm, T, M):
+    """Lines whose first stage is a prime beyond the register butterflies (it
+    reads the shared twiddle table at once), in blocks of several warps; a grid
+    of other line lengths is solved before each solve, so that shared memory
+    does not hold the right table from the solve before."""
+    rng = np.random.default_rng(sum(M))
+    grids = []
+    for m in ((60, 150, 126), M):
+        prod, ora = both(ffcm, T, **kw_of(tuple(float(n) for n in m), 1, m, M_G=2, R_c=min(m) / 2))
+        f = rng.standard_normal(ora.force_density.shape).astype(T) + T(0.3)
+        ora.force_density[:] = f
+        O.stokes_solve(ora)
+        grids.append((prod, f, ora.fluid_velocity))
+    for _ in range(3):
+        for prod, f, u in grids:
+            prod.set("FORCE_DENSITY", f)
+            ffcm.stokes_solve(prod)
+            assert rel_l2(prod.fluid_velocity, u) < UNITS * np.finfo(T).eps
