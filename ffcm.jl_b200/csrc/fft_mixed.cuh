@@ -264,7 +264,12 @@ __device__ __forceinline__ void mix_stage(const MixPlan& p, int s, int Ns, int l
 }
 
 // A stage of a prime radix above the register butterflies (up to 61): O(R^2),
-// every output sums over the inputs again.
+// every output sums over the inputs again. Outputs u > 0 of a butterfly without
+// twiddles sum the differences from its first value (the roots add up to zero):
+// a line's mean then drops out exactly, instead of leaving the rounding of R
+// table entries times the mean in the lowest modes, which the projector weighs
+// most (60 x 190 x 24, noise of deviation 1 about 0.3, Float64: 80 rounding
+// units of the velocities without, 4 with it).
 template <typename T, int NC, int KIND, typename S, typename D>
 __device__ __forceinline__ void mix_stage_prime(const MixPlan& p, int R, int s, int Ns, int lb, const cplx<T>* tw,
                                                 S src, D dst, bool inv) {
@@ -282,10 +287,11 @@ __device__ __forceinline__ void mix_stage_prime(const MixPlan& p, int R, int s, 
         const cplx<T>* a = src.p + c * src.cs + j * src.es + b;
         const auto as = m * src.es;
         const int de = (int)(((int64_t)u * root + (int64_t)k * p.step[s]) % size);
+        const cplx<T> base = k == 0 && u > 0 ? *a : cplx<T>{T(0), T(0)};
         cplx<T> acc{T(0), T(0)};
         int e = 0;
         for (int r = 0; r < R; ++r) {
-            acc = cadd(acc, cmul(*a, tw[e]));
+            acc = cadd(acc, cmul(csub(*a, base), tw[e]));
             a += as;
             e += de;
             if (e >= size) e -= size;

@@ -41,7 +41,7 @@ def test_stokes_solve_of_any_grid(ffcm, T, M):
 
 
 @pytest.mark.parametrize("T", [np.float32, np.float64])
-@pytest.mark.parametrize("M", [(64, 136, 32), (64, 32, 136), (48, 24, 228), (96, 204, 30), (96, 30, 114)])
+@pytest.mark.parametrize("M", [(64, 136, 32), (64, 32, 136), (60, 190, 24), (48, 24, 228), (96, 204, 30), (96, 30, 114)])
 def test_prime_first_stage_of_many_warps(ffcm, T, M):
     """Lines whose first stage is a prime beyond the register butterflies (it
     reads the shared twiddle table at once), in blocks of several warps; a grid
