@@ -328,9 +328,10 @@ struct EngineBase {
     virtual int forward_checkpoint(void* V, cudaStream_t s) = 0;
     virtual int adjoint(const void* lam, void* dY, void* dF, cudaStream_t s) = 0;
     virtual int residual(const void* V, const void* Vt, void* lam, double* J, cudaStream_t s) = 0;
-    virtual int ensure_adjoint() = 0;
+    virtual int ensure_adjoint(cudaStream_t s) = 0;
     virtual void* adj_buf(int which) = 0;  // 0 lambda, 1 dY, 2 dF, 3 target, 4 J (double)
-    virtual int ensure_real_grids() = 0;
+    // allocates the real grids on the first call and zeroes them on s
+    virtual int ensure_real_grids(cudaStream_t s) = 0;
     virtual bool uses_slab() const = 0;
     // the assembled solve works from particle lists that depend on the
     // positions only (ensure_lists)
@@ -1213,13 +1214,14 @@ struct Engine final : EngineBase {
 
     // The real force-density and velocity grids are needed only by the step
     // API and by the generic (non-slab) pipeline; they are allocated, zeroed,
-    // on first use.
-    int ensure_real_grids() override {
+    // on first use. On the stream of that use: the handle's streams do not wait
+    // for the legacy stream, where the zeroing could come after the first write.
+    int ensure_real_grids(cudaStream_t s) override {
         if (gf) return FFCM_OK;
         TRY(alloc(gf, 3 * (size_t)plane));
         TRY(alloc(gu, 3 * (size_t)plane));
-        CUDA_TRY(cudaMemset(gf, 0, 3 * (size_t)plane * sizeof(T)));
-        CUDA_TRY(cudaMemset(gu, 0, 3 * (size_t)plane * sizeof(T)));
+        CUDA_TRY(cudaMemsetAsync(gf, 0, 3 * (size_t)plane * sizeof(T), s));
+        CUDA_TRY(cudaMemsetAsync(gu, 0, 3 * (size_t)plane * sizeof(T), s));
         return FFCM_OK;
     }
 
@@ -1379,7 +1381,7 @@ struct Engine final : EngineBase {
             TRY(launch(h, sk.lists, (nslab + 7) / 8, 256, 0, s, (const vec4<T>*)Ys, (const int32_t*)off, sp, sg,
                        slab_lists, slab_counts));
         } else {
-            TRY(ensure_real_grids());
+            TRY(ensure_real_grids(s));
             if (pencil) TRY(pencil_lists(s));
         }
         lists_built = true;
@@ -1417,7 +1419,7 @@ struct Engine final : EngineBase {
         if (slab) {
             TRY(spread_to_spectrum(s, nullptr, build_lists));
         } else {
-            TRY(ensure_real_grids());
+            TRY(ensure_real_grids(s));
             if (build_lists) TRY(pencil_lists(s));
             TRY(pencil_spread(Fs, s));
         }
@@ -1643,7 +1645,7 @@ struct Engine final : EngineBase {
     // step API (spread_forces!): depends on Y_sorted/F_sorted only, as the
     // reference's, so it does not use the cell-list-driven slab kernel
     int spread_from(const vec4<T>* force, cudaStream_t s) {
-        TRY(ensure_real_grids());
+        TRY(ensure_real_grids(s));
         StageScope sc(h, FFCM_STAGE_SPREAD, s);
         CUDA_TRY(cudaMemsetAsync(gf, 0, 3 * (size_t)plane * sizeof(T), s));
         return launch(h, k_spread_atomic<T>, grid_for((int64_t)N * 32, 256, 148 * 64), 256,
@@ -1651,12 +1653,12 @@ struct Engine final : EngineBase {
     }
 
     int forward_checkpoint(void* V, cudaStream_t s) override {
-        TRY(ensure_adjoint());
+        TRY(ensure_adjoint(s));
         return solve(V, s, true);
     }
 
-    int ensure_adjoint() override {
-        TRY(ensure_real_grids());
+    int ensure_adjoint(cudaStream_t s) override {
+        TRY(ensure_real_grids(s));
         if (gpsi) return FFCM_OK;
         TRY(alloc(Ls, N));
         TRY(alloc(Lin, 3 * (size_t)N));
@@ -1665,8 +1667,8 @@ struct Engine final : EngineBase {
         TRY(alloc(Vt, 3 * (size_t)N));
         TRY(alloc(Jd, 1));
         TRY(alloc(gpsi, 3 * (size_t)plane));
-        CUDA_TRY(cudaMemset(Ls, 0, (size_t)N * sizeof(vec4<T>)));
-        CUDA_TRY(cudaMemset(gpsi, 0, 3 * (size_t)plane * sizeof(T)));
+        CUDA_TRY(cudaMemsetAsync(Ls, 0, (size_t)N * sizeof(vec4<T>), s));
+        CUDA_TRY(cudaMemsetAsync(gpsi, 0, 3 * (size_t)plane * sizeof(T), s));
         return FFCM_OK;
     }
 
@@ -1684,7 +1686,7 @@ struct Engine final : EngineBase {
     // sorted Y/F and the velocity grid u still in place): psi = L^-1 S lam,
     // then one stencil gather over (u, psi) and one pair pass.
     int adjoint(const void* lam, void* dY, void* dF, cudaStream_t s) override {
-        TRY(ensure_adjoint());
+        TRY(ensure_adjoint(s));
         {
             StageScope sc(h, FFCM_STAGE_CELL_LIST, s);
             TRY(launch(h, k_gather_forces<T>, grid_for(N, 256), 256, 0, s, N, (const int32_t*)perm,
@@ -1786,7 +1788,7 @@ struct Engine final : EngineBase {
     }
 
     int stokes(cudaStream_t s) override {
-        TRY(ensure_real_grids());
+        TRY(ensure_real_grids(s));
         return stokes_to(gu, s);
     }
 
@@ -1826,7 +1828,7 @@ struct Engine final : EngineBase {
     }
 
     int interp(void* V, cudaStream_t s) override {
-        TRY(ensure_real_grids());
+        TRY(ensure_real_grids(s));
         StageScope sc(h, FFCM_STAGE_INTERPOLATE, s);
         return launch(h, k_interpolate_warp<T>, grid_for((int64_t)N * 32, 256, 148 * 64), 256,
                       smem_stencil, s, N, (const vec4<T>*)Ys, (const int32_t*)perm,
@@ -1936,12 +1938,13 @@ void cg_release(ffcm_handle* h) {
 // while node whose body is one iteration captured on the handle's capture
 // stream. The graph holds only buffers of the handle, so it stays valid
 // across ffcm_set_positions calls (the particle lists are rebuilt outside it).
-int cg_build(ffcm_handle* h) {
+// The first solve runs on s, where the state is zeroed.
+int cg_build(ffcm_handle* h, cudaStream_t s) {
     auto& c = h->cg;
     const size_t bytes = 3 * (size_t)h->N * h->esize;
     for (void** p : {&c.x, &c.r, &c.p, &c.q}) CUDA_TRY(cudaMalloc(p, bytes));
     CUDA_TRY(cudaMalloc(&c.st, sizeof(CgState)));
-    CUDA_TRY(cudaMemset(c.st, 0, sizeof(CgState)));
+    CUDA_TRY(cudaMemsetAsync(c.st, 0, sizeof(CgState), s));
     CUDA_TRY(cudaMallocHost(&c.host, sizeof(CgState)));
     CUDA_TRY(cudaStreamCreateWithFlags(&c.cs, cudaStreamNonBlocking));
     CUDA_TRY(cudaGraphCreate(&c.graph, 0));
@@ -1981,9 +1984,9 @@ int cg_build(ffcm_handle* h) {
     return FFCM_OK;
 }
 
-int cg_prepare(ffcm_handle* h) {
+int cg_prepare(ffcm_handle* h, cudaStream_t s) {
     if (h->cg.exec) return FFCM_OK;
-    const int rc = cg_build(h);
+    const int rc = cg_build(h, s);
     if (rc != FFCM_OK) {
         const std::string msg = g_err;
         cg_release(h);
@@ -2527,7 +2530,7 @@ int ffcm_mobility_checkpoint(ffcm_handle* h, void* V, const void* Y, const void*
     DeviceGuard g(h->device);
     cudaStream_t s = h->pick(stream);
     EngineBase* e = h->eng.get();
-    TRY(e->ensure_adjoint());
+    TRY(e->ensure_adjoint(s));
     const size_t bytes = 3 * (size_t)h->N * h->esize;
     const void* Yd = Y;
     const void* Fd = F;
@@ -2594,7 +2597,7 @@ int ffcm_objective_gradient(ffcm_handle* h, double* J, void* dJdY, void* dJdF, v
     DeviceGuard g(h->device);
     cudaStream_t s = h->pick(stream);
     EngineBase* e = h->eng.get();
-    TRY(e->ensure_adjoint());
+    TRY(e->ensure_adjoint(s));
     const size_t bytes = 3 * (size_t)h->N * h->esize;
     const void *Yd = Y, *Fd = F, *Td = V_target;
     void *Vd = V, *dYd = dJdY, *dFd = dJdF;
@@ -2713,7 +2716,7 @@ int ffcm_cg_solve(ffcm_handle* h, void* F, const void* V, int32_t memory, double
                                                       : std::sqrt(std::numeric_limits<double>::epsilon());
     if (maxiter < 0) maxiter = (int32_t)std::min<int64_t>(3 * h->N, INT32_MAX);
     TRY(e->ensure_lists(s));
-    TRY(cg_prepare(h));
+    TRY(cg_prepare(h, s));
     auto& c = h->cg;
     const size_t bytes = 3 * (size_t)h->N * h->esize;
     const cudaMemcpyKind in = memory == FFCM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
@@ -2797,8 +2800,8 @@ int buffer_io(ffcm_handle* h, Engine<T>* e, int32_t which, void* ext, int64_t nb
     switch (which) {
         case FFCM_BUF_Y_WRAPPED: TRY(copy(e->Yw)); break;
         case FFCM_BUF_CELL_HASH: TRY(copy(e->key)); break;
-        case FFCM_BUF_FORCE_DENSITY: TRY(e->ensure_real_grids()); TRY(copy(e->gf)); break;
-        case FFCM_BUF_FLUID_VELOCITY: TRY(e->ensure_real_grids()); TRY(copy(e->gu)); break;
+        case FFCM_BUF_FORCE_DENSITY: TRY(e->ensure_real_grids(s)); TRY(copy(e->gf)); break;
+        case FFCM_BUF_FLUID_VELOCITY: TRY(e->ensure_real_grids(s)); TRY(copy(e->gu)); break;
         case FFCM_BUF_Y_SORTED:
         case FFCM_BUF_F_SORTED: {
             vec4<T>* dev = which == FFCM_BUF_Y_SORTED ? e->Ys : e->Fs;
@@ -3061,8 +3064,12 @@ int ffcm_batch_create(ffcm_batch** out, int32_t dtype, int64_t nsys, const doubl
         if (r != FFCM_OK) return bail(r);
         b->sys.push_back(h);
         if (!h->eng->uses_slab()) {
-            const int rr = h->eng->ensure_real_grids();   // before any capture
+            const int rr = h->eng->ensure_real_grids(h->stream);   // before any capture
             if (rr != FFCM_OK) return bail(rr);
+            if (cudaStreamSynchronize(h->stream) != cudaSuccess) {   // the batch's graph runs on other streams
+                fail(FFCM_ERR_CUDA, "zeroing the real grids");
+                return bail(FFCM_ERR_CUDA);
+            }
         }
         b->N.push_back(N[i]);
         b->yoff.push_back(acc);
