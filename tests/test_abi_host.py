@@ -101,3 +101,13 @@ def test_derived_scalars_bit_identical(ffcm, T, case, ratio):
 def test_create_requires_gpu_acceleration(ffcm):
     with pytest.raises(ffcm.ArgumentError):
         ffcm.FFCMConfig(np.float32, gpu_acceleration=False, **{k: v for k, v in BASE.items()})
+
+
+def test_build_is_the_same_every_time():
+    """The compiler splits its work by no number of threads: with
+    -split-compile one source gives libraries of different kernels."""
+    import subprocess
+    from conftest import ROOT
+    line = subprocess.run(["make", "-n", "-B", "-C", str(ROOT / "ffcm.jl_b200")], capture_output=True, text=True,
+                          check=True).stdout
+    assert "sm_100a" in line and "split-compile" not in line
