@@ -42,7 +42,10 @@ int fail(int code, const std::string& msg) {
     return code;
 }
 
+// The error is reported here and taken out of the runtime's last error, which
+// the next kernel launch would report as its own.
 int cuda_fail(cudaError_t e, const char* what) {
+    (void)cudaGetLastError();
     int code = (e == cudaErrorMemoryAllocation) ? FFCM_ERR_OOM : FFCM_ERR_CUDA;
     return fail(code, std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -575,6 +578,9 @@ struct Engine final : EngineBase {
     PencilGeom pg;
     int pen_bins = 0;
     int *pen_cnt = nullptr, *pen_off = nullptr, *pen_ent = nullptr, *pen_used = nullptr;
+    // counters that every finished cell list (pencil list) leaves zero: false
+    // while one is under way, so that the call after a failed launch zeroes them
+    bool cnt_zero = true, pen_zero = true;
 
     T *Yin = nullptr, *Fin = nullptr, *Vout = nullptr, *Yw = nullptr;
     int32_t *key = nullptr, *perm = nullptr, *cnt = nullptr, *off = nullptr, *tiles = nullptr;
@@ -1241,15 +1247,25 @@ struct Engine final : EngineBase {
 
     int wrap_hash(const void* Y, bool wrap, bool hash, cudaStream_t s, bool count) override {
         StageScope sc(h, FFCM_STAGE_CELL_LIST, s);
+        if (count) TRY(begin_count(s));
         return launch(h, k_wrap_hash<T>, grid_for(N, 256), 256, 0, s, N,
                       static_cast<const T*>(Y), Yw, key, L[0], L[1], L[2], d.inv_cell_size[0],
                       d.inv_cell_size[1], d.inv_cell_size[2], m0, m1, m2, h->d_err,
                       wrap ? 1 : 0, hash ? 1 : 0, count ? cnt : nullptr);
     }
 
+    int begin_count(cudaStream_t s) {
+        if (!cnt_zero) CUDA_TRY(cudaMemsetAsync(cnt, 0, (size_t)ncell * sizeof(int32_t), s));
+        cnt_zero = false;
+        return FFCM_OK;
+    }
+
     int sort(const void* F, cudaStream_t s, bool counted) override {
         StageScope sc(h, FFCM_STAGE_CELL_LIST, s);
-        if (!counted) TRY(launch(h, k_count_cells, grid_for(N, 256), 256, 0, s, N, (const int32_t*)key, cnt));
+        if (!counted) {
+            TRY(begin_count(s));
+            TRY(launch(h, k_count_cells, grid_for(N, 256), 256, 0, s, N, (const int32_t*)key, cnt));
+        }
         if (ncell <= SCAN_ONE_PASS) {
             TRY(launch(h, k_scan_one_pass, ntiles, SCAN_THREADS, 0, s, (const int32_t*)cnt, ncell, off));
         } else {
@@ -1260,6 +1276,7 @@ struct Engine final : EngineBase {
         }
         TRY(launch(h, k_scatter_cells, grid_for(N, 256), 256, 0, s, N, (const int32_t*)key,
                    (const int32_t*)off, cnt, scratch_i));
+        cnt_zero = true;
         return launch(h, k_rank_gather<T>, grid_for(N, 256), 256, 0, s, N, (const int32_t*)key,
                       (const int32_t*)off, (const int32_t*)scratch_i, perm, (const T*)Yw,
                       static_cast<const T*>(F), Ys, Fs);
@@ -1284,10 +1301,14 @@ struct Engine final : EngineBase {
     int pencil_lists(cudaStream_t s) {
         StageScope sc(h, FFCM_STAGE_SPREAD, s);
         const int npen = pg.nty * pg.ntz;
+        if (!pen_zero) CUDA_TRY(cudaMemsetAsync(pen_cnt, 0, ((size_t)pen_bins + 1) * sizeof(int), s));
+        pen_zero = false;
         TRY(launch(h, k_pencil_count<T>, grid_for((int64_t)N * PENCIL_SPLIT, 128), 128, 0, s, N, (const vec4<T>*)Ys, sp, pg, pen_cnt));
         TRY(launch(h, k_pencil_offsets, (npen + 7) / 8, 256, 0, s, npen, Mx, (const int*)pen_cnt, pen_off, pen_used));
-        return launch(h, k_pencil_scatter<T>, grid_for((int64_t)N * PENCIL_SPLIT, 128), 128, 0, s, N, (const vec4<T>*)Ys, sp, pg,
-                      (const int*)pen_off, pen_cnt, pen_ent, pen_used);
+        TRY(launch(h, k_pencil_scatter<T>, grid_for((int64_t)N * PENCIL_SPLIT, 128), 128, 0, s, N, (const vec4<T>*)Ys, sp, pg,
+                   (const int*)pen_off, pen_cnt, pen_ent, pen_used));
+        pen_zero = true;
+        return FFCM_OK;
     }
 
     int pencil_blocks() const { return (pg.nty * pg.ntz * pg.nseg + PENCIL_WARPS - 1) / PENCIL_WARPS; }
@@ -3052,6 +3073,7 @@ int ffcm_batch_create(ffcm_batch** out, int32_t dtype, int64_t nsys, const doubl
     b->nsys = nsys;
     b->esize = dtype == FFCM_FLOAT32 ? 4 : 8;
     auto bail = [&](int code) {
+        (void)cudaGetLastError();   // as in cuda_fail
         const std::string msg = g_err;
         batch_release(b);
         return fail(code, msg);
