@@ -1223,8 +1223,8 @@ struct Engine final : EngineBase {
     // on first use. On the stream of that use: the handle's streams do not wait
     // for the legacy stream, where the zeroing could come after the first write.
     int ensure_real_grids(cudaStream_t s) override {
-        if (gf) return FFCM_OK;
-        TRY(alloc(gf, 3 * (size_t)plane));
+        if (gu) return FFCM_OK;   // the last one made
+        if (!gf) TRY(alloc(gf, 3 * (size_t)plane));
         TRY(alloc(gu, 3 * (size_t)plane));
         CUDA_TRY(cudaMemsetAsync(gf, 0, 3 * (size_t)plane * sizeof(T), s));
         CUDA_TRY(cudaMemsetAsync(gu, 0, 3 * (size_t)plane * sizeof(T), s));
