@@ -543,7 +543,7 @@ struct Engine final : EngineBase {
     bool zmap_ok[5] = {false, false, false, false, false};
     CUtensorMap ymap[5];   // same, boxes for the TMA y pass
     bool ymap_ok[5] = {false, false, false, false, false};
-    int num_sms = 148;
+    int num_sms = 0;
     size_t smem_fx = 0, smem_fy = 0, smem_fz = 0;
     // spectrum held: planes (c, z) for z in the mzl planes of `spec` (all Mz
     // on one GPU, the rank's own z planes in a z-slab decomposition); the z
@@ -692,6 +692,13 @@ struct Engine final : EngineBase {
         cgc.ds_s = T(1) / (T(2) * s2);
         cgc.ds_S = T(1) / (T(2) * S2);
 
+        // (the launch shapes below are fitted to it)
+        {
+            int dev = 0;
+            CUDA_TRY(cudaGetDevice(&dev));
+            CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
+        }
+
         // FFT plans and launch shapes
         const bool xeven = (Mx % 2) == 0;
         TRY((mix_plan<T, false>(xeven ? Mx / 2 : Mx, xeven ? 2 : 1, 0, plan_x)));
@@ -826,11 +833,6 @@ struct Engine final : EngineBase {
             for (int i = 0; i < nc; ++i)
                 TRY(raise_smem_cap((const void*)z_kernel<T>(Mz, cand[i]), FastFft<T>::yz_smem(Mz, cand[i])));
             Bz = cand[nc - 1];
-        }
-        {
-            int dev = 0;
-            CUDA_TRY(cudaGetDevice(&dev));
-            CUDA_TRY(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev));
         }
         for (int B : {2, 4, 8, 16}) {
             if (fast_y && ypipe_kernel<T>(My, B) && hxp % B == 0 && ypipe_smem<T>(My, B) <= budget)
