@@ -701,14 +701,19 @@ struct Engine final : EngineBase {
 
         // FFT plans and launch shapes
         const bool xeven = (Mx % 2) == 0;
-        TRY((mix_plan<T, false>(xeven ? Mx / 2 : Mx, xeven ? 2 : 1, 0, plan_x)));
-        TRY((mix_plan<T, false>(My, 1, 0, plan_y)));
-        TRY((mix_plan<T, false>(Mz, 1, mix_fuse_radix<T>(), plan_z)));
+        const int nx = xeven ? Mx / 2 : Mx;   // complex line length along x
+        fast_x = xeven && fast_len(nx);
+        fast_y = fast_len(My);
+        fast_z = fast_len(Mz);
+        if (!fast_x) TRY((mix_plan<T, false>(nx, xeven ? 2 : 1, 0, plan_x)));
+        if (!fast_y) TRY((mix_plan<T, false>(My, 1, 0, plan_y)));
+        if (!fast_z) TRY((mix_plan<T, false>(Mz, 1, mix_fuse_radix<T>(), plan_z)));
         const size_t cs = sizeof(cplx<T>);
         const size_t budget = 200 * 1024;
-        if (2 * plan_x.n * cs > budget || 2 * My * cs > budget || 2 * 3 * (size_t)Mz * cs > budget)
+        if (2 * nx * cs > budget || 2 * My * cs > budget || 2 * 3 * (size_t)Mz * cs > budget)
             return fail(FFCM_ERR_UNSUPPORTED, "grid dimension too large for the shared-memory FFT");
-        // Lines per block: 128 bytes of a spectrum row (whole lines of every
+        // Mixed-radix passes, for the axes that launch them (every first use of a
+        // kernel loads it). Lines per block: 128 bytes of a spectrum row (whole lines of every
         // global access, shared-memory rows without bank conflicts; 64 for the
         // Float32 x rows, whose smaller blocks measured 105 against 120 us at
         // 240 x 200 x 160 before their loads were asynchronous), halved while a block would not leave room for a
@@ -755,13 +760,10 @@ struct Engine final : EngineBase {
             return FFCM_OK;
         };
         const int64_t xlines = xeven ? 3 * (int64_t)My * Mz : (3 * (int64_t)My * Mz + 1) / 2;
-        TRY(shape('x', plan_x, 1, xlines, 1, mx));
-        TRY(shape('y', plan_y, 1, nkx, 3 * (int64_t)Mz, my));
-        TRY(shape('z', plan_z, 3, nkx, My, mz));
+        if (!fast_x) TRY(shape('x', plan_x, 1, xlines, 1, mx));
+        if (!fast_y) TRY(shape('y', plan_y, 1, nkx, 3 * (int64_t)Mz, my));
+        if (!fast_z) TRY(shape('z', plan_z, 3, nkx, My, mz));
         smem_stencil = 8 * 3 * (size_t)MG * (2 * sizeof(T) + sizeof(int));
-        fast_x = xeven && fast_len(Mx / 2);
-        fast_y = fast_len(My);
-        fast_z = fast_len(Mz);
         if (fast_x) {
             lpb_fx = FastFft<T>::x_lpb(Mx / 2);
             smem_fx = FastFft<T>::x_smem(Mx / 2);
@@ -850,10 +852,13 @@ struct Engine final : EngineBase {
             if (fast_z && zpipe_kernel<T>(Mz, B) && zpitch % B == 0 && zpipe_smem<T>(Mz, B) <= budget)
                 TRY(raise_smem_cap((const void*)zpipe_kernel<T>(Mz, B), zpipe_smem<T>(Mz, B)));
         }
-        TRY(raise_smem_cap((const void*)(mx.longl ? k_fftm_x_r2c<T, true> : k_fftm_x_r2c<T, false>), mx.smem));
-        TRY(raise_smem_cap((const void*)(mx.longl ? k_fftm_x_c2r<T, true> : k_fftm_x_c2r<T, false>), mx.smem));
-        TRY(raise_smem_cap((const void*)(my.longl ? k_fftm_y<T, true> : k_fftm_y<T, false>), my.smem));
-        TRY(raise_smem_cap((const void*)(mz.longl ? k_fftm_z_stokes<T, true> : k_fftm_z_stokes<T, false>), mz.smem));
+        if (!fast_x) {
+            TRY(raise_smem_cap((const void*)(mx.longl ? k_fftm_x_r2c<T, true> : k_fftm_x_r2c<T, false>), mx.smem));
+            TRY(raise_smem_cap((const void*)(mx.longl ? k_fftm_x_c2r<T, true> : k_fftm_x_c2r<T, false>), mx.smem));
+        }
+        if (!fast_y) TRY(raise_smem_cap((const void*)(my.longl ? k_fftm_y<T, true> : k_fftm_y<T, false>), my.smem));
+        if (!fast_z)
+            TRY(raise_smem_cap((const void*)(mz.longl ? k_fftm_z_stokes<T, true> : k_fftm_z_stokes<T, false>), mz.smem));
         if (smem_stencil > 48 * 1024) {
             TRY(raise_smem_cap((const void*)k_spread_atomic<T>, smem_stencil));
             TRY(raise_smem_cap((const void*)k_interpolate_warp<T>, smem_stencil));
