@@ -903,11 +903,15 @@ struct Engine final : EngineBase {
         }
 
         if (pencil) {
-            TRY(alloc(partial, 3 * (size_t)N));
-            // one allocation (each costs 0.2 to 0.3 ms): counts, entries used, offsets, entries
+            // one allocation (each costs 0.2 to 0.3 ms): interpolation sums, then
+            // counts, entries used, offsets, entries
             const size_t noff = (size_t)pen_bins + (size_t)pg.nty * pg.ntz;
             const size_t nent = (size_t)N * pencil_reach(PENCIL_TY, MG, My) * pencil_reach(PENCIL_TZ, MG, Mz);
-            TRY(alloc(pen_cnt, (size_t)pen_bins + 1 + noff + nent));
+            const size_t sums = (3 * (size_t)N * sizeof(T) + 15) / 16 * 16;
+            unsigned char* base = nullptr;
+            TRY(alloc(base, sums + ((size_t)pen_bins + 1 + noff + nent) * sizeof(int)));
+            partial = reinterpret_cast<T*>(base);
+            pen_cnt = reinterpret_cast<int*>(base + sums);
             pen_used = pen_cnt + pen_bins;
             pen_off = pen_used + 1;
             pen_ent = pen_off + noff;

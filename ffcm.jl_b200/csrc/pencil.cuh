@@ -58,8 +58,11 @@ struct PencilReach {
     __device__ __forceinline__ int tile(int i) const { return i < n1 ? t0 + i : i - n1; }
 };
 
-// Most pencils one particle can reach along an axis (tiles of ts rows).
-inline int pencil_reach(int ts, int MG, int M) { return std::min((M + ts - 1) / ts, (MG + ts - 2) / ts + 2); }
+// Most pencils one particle can reach along an axis (tiles of ts rows): one more
+// where the last tile is a short one.
+inline int pencil_reach(int ts, int MG, int M) {
+    return std::min((M + ts - 1) / ts, (MG + ts - 2) / ts + (M % ts == 0 ? 1 : 2));
+}
 
 // First x point of a stencil, in [0, Mx).
 template <typename T>
