@@ -578,6 +578,8 @@ struct Engine final : EngineBase {
     PencilGeom pg;
     int pen_bins = 0;
     int *pen_cnt = nullptr, *pen_off = nullptr, *pen_ent = nullptr, *pen_used = nullptr;
+    PencilTasks pen_tasks{};
+    int pen_more = 0;   // most further parts
     // counters that every finished cell list (pencil list) leaves zero: false
     // while one is under way, so that the call after a failed launch zeroes them
     bool cnt_zero = true, pen_zero = true;
@@ -808,6 +810,16 @@ struct Engine final : EngineBase {
             const int want = std::max(1, std::min((num_sms * 24 + npen - 1) / npen, Mx / (4 * MG)));
             pg.seg = ((Mx + want - 1) / want + piece - 1) / piece * piece;
             pg.nseg = (Mx + pg.seg - 1) / pg.seg;
+            // a warp's entries: at most twice what a segment of a uniform
+            // suspension holds (M_G + 7 by M_G + 3 rows reach a pencil's 8 by 4),
+            // so that such a one is hardly split, and not below four batches.
+            // Spread + interpolation of clusters at 256^3, M_G = 10, N =
+            // 186,510, us by that factor: 804 (1.5), 837 (2), 933 (3), 1095 (5),
+            // 1517 (never split), Float64 1336, 1386, 1576, 1954, 2492; uniform
+            // positions 609 to 619 and 1058 to 1065 with any of them
+            const double mean = (double)N * (MG + PENCIL_TY - 1) * (MG + PENCIL_TZ - 1) / (PENCIL_TY * PENCIL_TZ) *
+                                (1.0 + (MG - 1.0) / pg.seg) / ((double)npen * pg.nseg);
+            pg.part = (int)std::max(128.0, 2.0 * mean);
             TRY(raise_smem_cap((const void*)pk.spread, pk.smem));
             TRY(raise_smem_cap((const void*)pk.interp, pk.smem_interp));
         }
@@ -904,18 +916,24 @@ struct Engine final : EngineBase {
 
         if (pencil) {
             // one allocation (each costs 0.2 to 0.3 ms): interpolation sums, then
-            // counts, entries used, offsets, entries
+            // further parts, counts, entries used and parts used, offsets, parts, entries
             const size_t noff = (size_t)pen_bins + (size_t)pg.nty * pg.ntz;
             const size_t nent = (size_t)N * pencil_reach(PENCIL_TY, MG, My) * pencil_reach(PENCIL_TZ, MG, Mz);
-            const size_t sums = (3 * (size_t)N * sizeof(T) + 15) / 16 * 16;
+            // an entry's stencil lies in two segments, or three with a short last one
+            pen_more = (int)((pg.nseg == 1 || Mx % pg.seg == 0 ? 2 : 3) * nent / pg.part) + 1;
+            const size_t nseg = (size_t)pg.nty * pg.ntz * pg.nseg;
+            const size_t sums = (3 * (size_t)N * sizeof(T) + 15) / 16 * 16, more = (size_t)pen_more * sizeof(int2);
             unsigned char* base = nullptr;
-            TRY(alloc(base, sums + ((size_t)pen_bins + 1 + noff + nent) * sizeof(int)));
+            TRY(alloc(base, sums + more + ((size_t)pen_bins + 2 + noff + nseg + nent) * sizeof(int)));
             partial = reinterpret_cast<T*>(base);
-            pen_cnt = reinterpret_cast<int*>(base + sums);
+            pen_tasks.more = reinterpret_cast<int2*>(base + sums);
+            pen_cnt = reinterpret_cast<int*>(base + sums + more);
             pen_used = pen_cnt + pen_bins;
-            pen_off = pen_used + 1;
-            pen_ent = pen_off + noff;
-            CUDA_TRY(cudaMemset(pen_cnt, 0, ((size_t)pen_bins + 1) * sizeof(int)));
+            pen_tasks.nmore = pen_used + 1;
+            pen_off = pen_used + 2;
+            pen_tasks.parts = pen_off + noff;
+            pen_ent = pen_tasks.parts + nseg;
+            CUDA_TRY(cudaMemset(pen_cnt, 0, ((size_t)pen_bins + 2) * sizeof(int)));
         }
 
         // zero-initialised grids and cell list (src/config.jl:443-448)
@@ -1314,29 +1332,31 @@ struct Engine final : EngineBase {
         const int npen = pg.nty * pg.ntz;
         if (!pen_zero) CUDA_TRY(cudaMemsetAsync(pen_cnt, 0, ((size_t)pen_bins + 1) * sizeof(int), s));
         pen_zero = false;
-        TRY(launch(h, k_pencil_count<T>, grid_for((int64_t)N * PENCIL_SPLIT, 128), 128, 0, s, N, (const vec4<T>*)Ys, sp, pg, pen_cnt));
-        TRY(launch(h, k_pencil_offsets, (npen + 7) / 8, 256, 0, s, npen, Mx, (const int*)pen_cnt, pen_off, pen_used));
+        TRY(launch(h, k_pencil_count<T>, grid_for((int64_t)N * PENCIL_SPLIT, 128), 128, 0, s, N, (const vec4<T>*)Ys, sp, pg, pen_cnt, pen_tasks));
+        TRY(launch(h, k_pencil_offsets, (npen + 7) / 8, 256, 0, s, npen, Mx, MG, pg, (const int*)pen_cnt, pen_off, pen_used, pen_tasks));
         TRY(launch(h, k_pencil_scatter<T>, grid_for((int64_t)N * PENCIL_SPLIT, 128), 128, 0, s, N, (const vec4<T>*)Ys, sp, pg,
                    (const int*)pen_off, pen_cnt, pen_ent, pen_used));
         pen_zero = true;
         return FFCM_OK;
     }
 
-    int pencil_blocks() const { return (pg.nty * pg.ntz * pg.nseg + PENCIL_WARPS - 1) / PENCIL_WARPS; }
+    // a warp for every segment and for every further part there can be
+    int pencil_blocks() const { return (pg.nty * pg.ntz * pg.nseg + pen_more + PENCIL_WARPS - 1) / PENCIL_WARPS; }
 
     // forces -> force density on the real grid (every point written); `partial`
     // zeroed for the interpolation
     int pencil_spread(const vec4<T>* force, cudaStream_t s) {
         StageScope sc(h, FFCM_STAGE_SPREAD, s);
+        TRY(launch(h, k_pencil_zero<T>, std::min(pen_more, 2 * num_sms), 256, 0, s, sp, pg, pen_tasks, gf));
         return launch(h, pk.spread, pencil_blocks(), 32 * PENCIL_WARPS, pk.smem, s, (const vec4<T>*)Ys, force, sp, pg,
-                      (const int*)pen_off, (const int*)pen_ent, gf, partial, 3 * (int64_t)N);
+                      (const int*)pen_off, (const int*)pen_ent, pen_tasks, gf, partial, 3 * (int64_t)N);
     }
 
     // velocities gu -> h^-3 V in sorted order in `partial`
     int pencil_interp(cudaStream_t s) {
         StageScope sc(h, FFCM_STAGE_INTERPOLATE, s);
         return launch(h, pk.interp, pencil_blocks(), 32 * PENCIL_WARPS, pk.smem_interp, s, (const vec4<T>*)Ys, sp, pg,
-                      (const int*)pen_off, (const int*)pen_ent, (const T*)gu, partial);
+                      (const int*)pen_off, (const int*)pen_ent, pen_tasks, (const T*)gu, partial);
     }
 
     // Hot path of the assembled operator: spread straight into the x-transformed

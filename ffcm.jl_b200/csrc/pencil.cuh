@@ -25,9 +25,10 @@
 // shared memory): per entry and pencil 2.5 M_G two-wide multiply-adds and as
 // many instructions again for its weights, loads and the walk; of the
 // (M_G + 7)(M_G + 3) rows its pencils hold, an entry uses M_G^2. N = 186,510,
-// 256^3, M_G = 10, Float32: spread 311 us (the lists 35 us more) against 690 us
+// 256^3, M_G = 10, Float32: spread 300 us (the lists 35 us more) against 700 us
 // with global atomics, which run at one 32-byte sector per L2 slice and clock;
-// interpolation 343 against 675 us, where every warp read 20 KB through L1.
+// interpolation 275 against 675 us, where every warp read 20 KB through L1
+// (Float64: 475 and 546 against 1035 and 775 us).
 #pragma once
 
 #include "common.cuh"
@@ -43,6 +44,17 @@ constexpr int PENCIL_WARPS = 2;               // warps per block (they share not
 struct PencilGeom {
     int nty, ntz;    // pencils along y and z
     int nseg, seg;   // segments of a row, points per segment
+    int part;        // most entries a warp walks: longer segments go to several
+};
+
+// The warps' tasks: one per segment (its part 0), and the further parts of the
+// segments whose entries exceed PencilGeom::part, so that a cluster's entries,
+// which lie in few segments, do not keep a few warps busy alone. Parts of a
+// segment add their sums to its grid points, zeroed by k_pencil_zero.
+struct PencilTasks {
+    int* parts;   // per segment: parts, 1 or more
+    int2* more;   // (segment, part > 0)
+    int* nmore;
 };
 
 // Pencils along one axis (tiles of TS rows out of M) that the rows s .. s + MG - 1
@@ -93,16 +105,30 @@ __device__ __forceinline__ void pencil_bins(int n_part, const vec4<T>* __restric
 
 template <typename T>
 __global__ void k_pencil_count(int n_part, const vec4<T>* __restrict__ Ys, StencilParams<T> p, PencilGeom g,
-                               int* __restrict__ cnt) {
+                               int* __restrict__ cnt, PencilTasks tasks) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *tasks.nmore = 0;
     pencil_bins(n_part, Ys, p, g, [&](int, int pen, int x) { atomicAdd(&cnt[pen * p.Mx + x], 1); });
+}
+
+// The entries of a pencil whose stencil reaches its points [xs, xe), from its bin
+// boundaries: first points xs - MG + 1 .. xe - 1, those below 0 from the row's
+// end (entries a0 .. a0 + na - 1, the image one period lower), then b0 .. b0 +
+// nb - 1.
+__device__ __forceinline__ void pencil_range(const int* bins, int xs, int xe, int Mx, int MG, int& a0,
+                                             int& na, int& b0, int& nb) {
+    const int lo = xs - MG + 1;
+    a0 = lo < 0 ? bins[lo + Mx] : 0;
+    na = lo < 0 ? bins[Mx] - a0 : 0;
+    b0 = bins[max(lo, 0)];
+    nb = bins[xe] - b0;
 }
 
 // One warp per pencil: offsets of its Mx + 1 bin boundaries from the bin counts.
 // The pencils take their parts of the entry list in any order (one atomic
-// each), so no scan across pencils is needed. *used is zero before;
-// k_pencil_scatter resets it.
-__global__ void k_pencil_offsets(int npen, int Mx, const int* __restrict__ cnt, int* __restrict__ off,
-                                 int* __restrict__ used) {
+// each), so no scan across pencils is needed. *used and *tasks.nmore are zero
+// before (k_pencil_scatter resets the one, k_pencil_count the other).
+__global__ void k_pencil_offsets(int npen, int Mx, int MG, PencilGeom g, const int* __restrict__ cnt,
+                                 int* __restrict__ off, int* __restrict__ used, PencilTasks tasks) {
     const int lane = threadIdx.x & 31;
     const int pen = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (pen >= npen) return;   // whole warps
@@ -126,6 +152,37 @@ __global__ void k_pencil_offsets(int npen, int Mx, const int* __restrict__ cnt, 
         base += __shfl_sync(0xffffffffu, s, 31);
     }
     if (lane == 0) o[Mx] = base;
+    __syncwarp();
+    for (int q = lane; q < g.nseg; q += 32) {
+        int a0, na, b0, nb;
+        pencil_range(o, q * g.seg, min((q + 1) * g.seg, Mx), Mx, MG, a0, na, b0, nb);
+        const int n = max(1, (int)(((int64_t)na + nb + g.part - 1) / g.part)), seg = pen * g.nseg + q;
+        tasks.parts[seg] = n;
+        if (n > 1) {
+            const int at = atomicAdd(tasks.nmore, n - 1);
+            for (int i = 1; i < n; ++i) tasks.more[at + i - 1] = make_int2(seg, i);
+        }
+    }
+}
+
+// Zeroes the grid points of the segments that several warps share.
+template <typename T>
+__global__ void k_pencil_zero(StencilParams<T> p, PencilGeom g, PencilTasks tasks, T* __restrict__ grid) {
+    const int n = *tasks.nmore;
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        const int2 t = tasks.more[i];
+        if (t.y != 1) continue;   // once a segment
+        const int pen = t.x / g.nseg, xs = (t.x - pen * g.nseg) * g.seg, w = min(g.seg, p.Mx - xs);
+        const int y0r = pen % g.nty * PENCIL_TY, z0r = pen / g.nty * PENCIL_TZ;
+        const int ny = min(PENCIL_TY, p.My - y0r), nz = min(PENCIL_TZ, p.Mz - z0r);
+        for (int e = threadIdx.x; e < 3 * ny * nz * w; e += blockDim.x) {
+            int r = e / w;
+            const int x = e - r * w, c = r / (ny * nz);
+            r -= c * ny * nz;
+            const int z = r / ny, y = r - z * ny;
+            grid[(((int64_t)c * p.Mz + z0r + z) * p.My + y0r + y) * p.Mx + xs + x] = T(0);
+        }
+    }
 }
 
 // cnt is consumed (left zero for the next count), as is *used.
@@ -248,13 +305,42 @@ struct PencilRows {
             for (int b = 0; b < PENCIL_TY; b += GROUP)
                 f(d * PENCIL_TY + b + lane / XC, b < ny && d < nz, base + d * zs + b * p.Mx);
     }
+    // staged columns added to the grid, where `on` (rolled: the code of 96 atomics
+    // beside the stores cost every spread a tenth of its time)
+    __device__ __forceinline__ void add(const StencilParams<T>& p, int lane, bool on, int64_t plane, T* out,
+                                     const T (*stage)[32][XC + 1]) const {
+        if (!on) return;
+#pragma unroll 1
+        for (int i = 0; i < 3 * PENCIL_TZ * PENCIL_TY; i += GROUP) {
+            const int c = i / (PENCIL_TZ * PENCIL_TY), d = i / PENCIL_TY % PENCIL_TZ, b = i % PENCIL_TY;
+            if (b < ny && d < nz)
+                atomicAdd(out + c * plane + base + ((int64_t)d * p.My + b) * p.Mx,
+                          stage[c][d * PENCIL_TY + b + lane / XC][lane % XC]);
+        }
+    }
 };
+
+// The warp's task: segment and part of it; false beyond the last one.
+__device__ __forceinline__ bool pencil_task(const PencilGeom& g, const PencilTasks& tasks, int& seg, int& part,
+                                            int& parts) {
+    const int nseg = g.nty * g.ntz * g.nseg, task = blockIdx.x * PENCIL_WARPS + (threadIdx.x >> 5);
+    seg = task;
+    part = 0;
+    if (task >= nseg) {
+        if (task - nseg >= *tasks.nmore) return false;
+        const int2 t = tasks.more[task - nseg];
+        seg = t.x;
+        part = t.y;
+    }
+    parts = tasks.parts[seg];
+    return true;
+}
 
 template <typename T, int MGT>
 __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 10 : 6)
     k_pencil_spread(const vec4<T>* __restrict__ Ys, const vec4<T>* __restrict__ Fs, const __grid_constant__
                     StencilParams<T> p, PencilGeom g, const int* __restrict__ off, const int* __restrict__ ent,
-                    T* __restrict__ grid, T* __restrict__ Vs, int64_t nvs) {
+                    PencilTasks tasks, T* __restrict__ grid, T* __restrict__ Vs, int64_t nvs) {
     using Warp = PencilWarp<T, MGT>;
     constexpr int XC = Warp::XC;
     zero_sums(Vs, nvs);
@@ -262,40 +348,43 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 10 : 6)
     const int lane = threadIdx.x & 31;
     PencilSpreadWarp<T, MGT>& S = reinterpret_cast<PencilSpreadWarp<T, MGT>*>(pencil_smem)[threadIdx.x >> 5];
     Warp& W = S.w;
-    const int task = blockIdx.x * PENCIL_WARPS + (threadIdx.x >> 5);
-    if (task >= g.nty * g.ntz * g.nseg) return;   // whole warps
-    const int pen = task / g.nseg;
-    const int xs = (task - pen * g.nseg) * g.seg, xe = min(xs + g.seg, p.Mx);
+    int seg, part, parts;
+    if (!pencil_task(g, tasks, seg, part, parts)) return;   // whole warps
+    const int pen = seg / g.nseg;
+    const int xs = (seg - pen * g.nseg) * g.seg, xe = min(xs + g.seg, p.Mx);
     const int y0r = pen % g.nty * PENCIL_TY, z0r = pen / g.nty * PENCIL_TZ;
     const PencilRows<T, MGT> rows(p, y0r, z0r, lane);
     const int64_t plane = (int64_t)p.Mx * p.My * p.Mz;
-    // entries whose stencil reaches [xs, xe): first points lo .. xe - 1, those
-    // below 0 from the row's end (the image one period lower)
-    const int lo = xs - p.MG + 1;
-    const int* bins = off + (int64_t)pen * (p.Mx + 1);
-    const int a0 = lo < 0 ? bins[lo + p.Mx] : 0, na = lo < 0 ? bins[p.Mx] - a0 : 0;
-    const int b0 = bins[max(lo, 0)], total = na + bins[xe] - b0;
+    int a0, na, b0, nb;
+    pencil_range(off + (int64_t)pen * (p.Mx + 1), xs, xe, p.Mx, p.MG, a0, na, b0, nb);
+    // the part's entries; parts > 1: the points they reach, added to the grid
+    const int first = (int)((int64_t)(na + nb) * part / parts), total = (int)((int64_t)(na + nb) * (part + 1) / parts);
+    int xend = xe;
     pair2<T> acc[3][MGT / 2];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
         for (int k = 0; k < MGT / 2; ++k) acc[c][k] = pair2<T>(T(0), T(0));
-    int X = lo;   // x of acc[.][0]
+    int X = xs - p.MG + 1;   // x of acc[.][0]
     auto advance = [&] {
         if (X >= xs) {
             const int col = (X - xs) % XC;
 #pragma unroll
             for (int c = 0; c < 3; ++c) W.stage[c][lane][col] = acc[c][0].x();
-            if (col == XC - 1 || X == xe - 1) {
+            if (col == XC - 1 || X == xend - 1) {
                 __syncwarp();
                 const int cc = lane % XC;
                 T* out = grid + (X - col + cc);
-                rows.each(p, lane, [&](int r, bool in, int64_t at) {
-                    if (in && cc <= col) {
+                if (parts == 1) {
+                    rows.each(p, lane, [&](int r, bool in, int64_t at) {
+                        if (in && cc <= col) {
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) out[c * plane + at] = W.stage[c][r][cc];
-                    }
-                });
+                            for (int c = 0; c < 3; ++c) out[c * plane + at] = W.stage[c][r][cc];
+                        }
+                    });
+                } else {
+                    rows.add(p, lane, cc <= col, plane, out, W.stage);
+                }
                 __syncwarp();
             }
         }
@@ -318,8 +407,12 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 10 : 6)
             xn = pencil_first(p, yn.x) - (i < na ? p.Mx : 0);
         }
     };
-    fetch(lane);
-    for (int base = 0; base < total; base += 32) {
+    fetch(first + lane);
+    if (parts > 1) {   // from the chunk of the first entry's first point
+        const int x = __shfl_sync(0xffffffffu, xn, 0);
+        X = x < xs ? x : x - (x - xs) % XC;
+    }
+    for (int base = first; base < total; base += 32) {
         const int n = min(32, total - base);
         if (lane < n) {
             W.x0[lane] = xn;
@@ -347,7 +440,8 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 10 : 6)
         }
         __syncwarp();
     }
-    while (X < xe) advance();
+    if (parts > 1) xend = min(xe, X + MGT);
+    while (X < xend) advance();
 }
 
 // Sums for entries in groups: every lane leaves its part of an
@@ -364,8 +458,8 @@ struct PencilInterpWarp {
 template <typename T, int MGT>
 __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 8 : 5)
     k_pencil_interp(const vec4<T>* __restrict__ Ys, const __grid_constant__ StencilParams<T> p, PencilGeom g,
-                    const int* __restrict__ off, const int* __restrict__ ent, const T* __restrict__ grid,
-                    T* __restrict__ Vs) {
+                    const int* __restrict__ off, const int* __restrict__ ent, PencilTasks tasks,
+                    const T* __restrict__ grid, T* __restrict__ Vs) {
     using Warp = PencilWarp<T, MGT>;
     constexpr int XC = Warp::XC;
     extern __shared__ __align__(32) unsigned char pencil_smem[];
@@ -373,17 +467,18 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 8 : 5)
     PencilInterpWarp<T, MGT>& I = reinterpret_cast<PencilInterpWarp<T, MGT>*>(pencil_smem)[threadIdx.x >> 5];
     Warp& W = I.w;
     constexpr int SUM_GROUP = PencilInterpWarp<T, MGT>::SUM_GROUP;
-    const int task = blockIdx.x * PENCIL_WARPS + (threadIdx.x >> 5);
-    if (task >= g.nty * g.ntz * g.nseg) return;   // whole warps
-    const int pen = task / g.nseg;
-    const int xs = (task - pen * g.nseg) * g.seg, xe = min(xs + g.seg, p.Mx);
+    int seg, part, parts;
+    if (!pencil_task(g, tasks, seg, part, parts)) return;   // whole warps
+    const int pen = seg / g.nseg;
+    const int xs = (seg - pen * g.nseg) * g.seg, xe = min(xs + g.seg, p.Mx);
     const int y0r = pen % g.nty * PENCIL_TY, z0r = pen / g.nty * PENCIL_TZ;
     const PencilRows<T, MGT> rows(p, y0r, z0r, lane);
     const int64_t plane = (int64_t)p.Mx * p.My * p.Mz;
     // every entry belongs to the segment its first point lies in
     const int* bins = off + (int64_t)pen * (p.Mx + 1);
-    const int b0 = bins[xs], total = bins[xe] - b0;
-    if (total == 0) return;
+    const int b0 = bins[xs], all = bins[xe] - b0;
+    const int first = (int)((int64_t)all * part / parts), total = (int)((int64_t)all * (part + 1) / parts);
+    if (first == total) return;
     pair2<T> u[3][MGT / 2];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
@@ -401,8 +496,18 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 8 : 5)
             ++i;
         });
     };
-    int X = xs - MGT;    // x of u[.][0]
-    load_chunk(xs);
+    int sn = 0;
+    vec4<T> yn{};
+    auto fetch = [&](int i) {
+        if (i < total) {
+            sn = ent[b0 + i];
+            yn = Ys[sn];
+        }
+    };
+    fetch(first + lane);
+    // x of u[.][0]: the first column to come is the chunk of the first entry's first point
+    int X = xs - MGT + (pencil_first(p, __shfl_sync(0xffffffffu, yn.x, 0)) - xs) / XC * XC;
+    load_chunk(X + MGT);
     auto advance = [&] {   // shifts column X + MGT in
         const int col = (X + MGT - xs) % XC;
         if (col == 0) {
@@ -423,16 +528,7 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 8 : 5)
         }
         ++X;
     };
-    int sn = 0;
-    vec4<T> yn{};
-    auto fetch = [&](int i) {
-        if (i < total) {
-            sn = ent[b0 + i];
-            yn = Ys[sn];
-        }
-    };
-    fetch(lane);
-    for (int base = 0; base < total; base += 32) {
+    for (int base = first; base < total; base += 32) {
         const int n = min(32, total - base);
         if (lane < n) {
             I.s[lane] = sn;
@@ -475,10 +571,10 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 8 : 5)
 
 template <typename T>
 using PencilSpreadKernel = void (*)(const vec4<T>*, const vec4<T>*, const StencilParams<T>, PencilGeom, const int*,
-                                    const int*, T*, T*, int64_t);
+                                    const int*, PencilTasks, T*, T*, int64_t);
 template <typename T>
 using PencilInterpKernel = void (*)(const vec4<T>*, const StencilParams<T>, PencilGeom, const int*, const int*,
-                                    const T*, T*);
+                                    PencilTasks, const T*, T*);
 
 template <typename T>
 struct PencilKernels {

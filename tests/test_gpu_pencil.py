@@ -120,3 +120,53 @@ def test_pencil_batch_under_capture(ffcm, forced):
         ora = O.OracleConfig(T, kernel_widths_ratio=2.0, M_G=9, viscosity=1.0, **s)
         for f, v in zip(fs, vs):
             assert rel_l2(v, O.apply(ora, Y, f)) < TOL[T]
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+@pytest.mark.parametrize("M,MG,N", [((40, 30, 50), 7, 3000), ((96, 40, 36), 12, 4000), ((130, 24, 20), 5, 2500),
+                                    ((33, 17, 9), 9, 1500)])
+def test_pencils_shared_by_several_warps(ffcm, forced, T, M, MG, N):
+    """Clusters whose segments hold more entries than one warp walks:
+    every solve of a configuration, on new and on kept lists and in the adjoint,
+    against the warp-per-particle grid steps."""
+    L = tuple(0.6 * m for m in M)
+    rng = np.random.default_rng(N)
+    Y = np.concatenate([np.array(c) * np.array(L) + 1.2 * rng.standard_normal((N // 2, 3))
+                        for c in ((0.4, 0.5, 0.3), (0.98, 0.02, 0.97))]).astype(T)
+    F, lam = (rng.standard_normal((N, 3)).astype(T) for _ in range(2))
+    got = []
+    for mode in "10":
+        forced.setenv("FFCM_PENCIL", mode)
+        cfg = ffcm.FFCMConfig(T, **kw_of(L, N, M, M_G=MG, R_c=0.3 * min(L)))
+        res = [ffcm.mobility(np.empty_like(Y), cfg, Y, F) for _ in range(2)]
+        A = ffcm.FFCMMobility(cfg, Y)
+        res += [A @ F, A @ lam]
+        V, pull = ffcm.rrule_mobility(cfg, Y, F)
+        res += [V, *pull(lam)]
+        got.append(res)
+    for i, (a, b) in enumerate(zip(*got)):
+        assert rel_l2(a, b) < TOL[T] * (10 if i > 4 else 1)   # (gradients cancel, as above)
+
+
+@pytest.mark.parametrize("T", [np.float32, np.float64])
+@pytest.mark.parametrize("overlap", ["0", "1"])
+def test_pencil_solve_with_the_correction_beside_it(ffcm, forced, T, overlap):
+    """Both orders of the pair correction, from host arrays and from device
+    arrays on a caller's stream, the first solve of a configuration included."""
+    import torch
+    forced.setenv("FFCM_OVERLAP_PAIRS", overlap)
+    M, N = (50, 36, 42), 700
+    L = tuple(0.55 * m for m in M)
+    kw = kw_of(L, N, M, M_G=9, R_c=3.0)
+    prod, ora = both(ffcm, T, **kw)
+    Y, F = _inputs(T, L, N, "uniform", 17)
+    ref = O.apply(ora, Y, F)
+    for _ in range(3):
+        assert rel_l2(ffcm.mobility(np.empty_like(Y), prod, Y, F), ref) < TOL[T]
+    cfg, s = ffcm.FFCMConfig(T, **kw), torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        Yd, Fd = torch.from_numpy(Y).cuda(), torch.from_numpy(F).cuda()
+        for _ in range(3):
+            V = ffcm.mobility(torch.empty_like(Fd), cfg, Yd, Fd)
+            s.synchronize()
+            assert rel_l2(V.cpu().numpy(), ref) < TOL[T]
