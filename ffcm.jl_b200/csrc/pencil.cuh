@@ -19,7 +19,11 @@
 //
 // The weights of 32 entries at a time are evaluated by one lane per entry and
 // read as broadcasts; the weight of a point is
-// [gx (a0 + a2 r2x)] (gy gz) + [a2 gx] (gy gz (r2y + r2z)).
+// gx [(a0 + a2 r2x) (gy gz) + gy gz (a2 r2y + a2 r2z)]: two instructions for two
+// points, with 1.34e-7 of the weights lost to Float32 rounding (M_G = 10) where
+// (a0 + a2 r^2) gx (gy gz), of three, loses 1.29e-7. The velocities of the record
+// configuration (N = 186,510) are 2.49e-7 off in Float32 (mean of five seeds)
+// against 2.34e-7 with a warp per particle, in Float64 5.34e-16 against 5.13e-16.
 //
 // What bounds it: instruction issue (ncu: 66% of issue slots, the rest waits on
 // shared memory): per entry and pencil 2.5 M_G two-wide multiply-adds and as
@@ -27,8 +31,8 @@
 // (M_G + 7)(M_G + 3) rows its pencils hold, an entry uses M_G^2. N = 186,510,
 // 256^3, M_G = 10, Float32: spread 300 us (the lists 35 us more) against 700 us
 // with global atomics, which run at one 32-byte sector per L2 slice and clock;
-// interpolation 275 against 675 us, where every warp read 20 KB through L1
-// (Float64: 475 and 546 against 1035 and 775 us).
+// interpolation 273 against 675 us, where every warp read 20 KB through L1
+// (Float64: 475 and 534 against 1035 and 775 us).
 #pragma once
 
 #include "common.cuh"
@@ -206,7 +210,8 @@ struct PencilWarp {
     static constexpr int PER = 16 / (int)sizeof(T);
     static constexpr int CH = (2 * MGT + PER - 1) / PER;
     static constexpr int SW = (CH | 1) * PER;
-    T wx[32][SW];                        // gx (a0 + a2 r2x) of the M_G points, then a2 gx
+    T wx[32][SW];                        // gx of the M_G points, then a0 + a2 r2x
+    // (ry, rz: a2 r2y, a2 r2z)
     T gy[PENCIL_TY][33], ry[PENCIL_TY][33], gz[PENCIL_TZ][33], rz[PENCIL_TZ][33];
     T stage[3][32][XC + 1];
     int x0[32];                          // first x point, relative to the segment's row
@@ -238,8 +243,8 @@ __device__ __forceinline__ void pencil_put(const StencilParams<T>& p, PencilWarp
             T gx, r2;
             weight(sx + k, y.x, gx, r2);
             if (k >= p.MG) gx = T(0);
-            W.wx[lane][k] = gx * (p.a0 + p.a2 * r2);
-            W.wx[lane][MGT + k] = p.a2 * gx;
+            W.wx[lane][k] = gx;
+            W.wx[lane][MGT + k] = p.a0 + p.a2 * r2;
         }
 #pragma unroll 2
         for (int b = 0; b < PENCIL_TY; ++b) {
@@ -248,7 +253,7 @@ __device__ __forceinline__ void pencil_put(const StencilParams<T>& p, PencilWarp
             weight(sy + d, y.y, g, r2);
             const bool hit = d < p.MG && y0r + b < p.My;
             W.gy[b][lane] = hit ? g : T(0);
-            W.ry[b][lane] = hit ? r2 : T(0);
+            W.ry[b][lane] = hit ? p.a2 * r2 : T(0);
         }
 #pragma unroll 2
         for (int b = 0; b < PENCIL_TZ; ++b) {
@@ -257,7 +262,7 @@ __device__ __forceinline__ void pencil_put(const StencilParams<T>& p, PencilWarp
             weight(sz + d, y.z, g, r2);
             const bool hit = d < p.MG && z0r + b < p.Mz;
             W.gz[b][lane] = hit ? g : T(0);
-            W.rz[b][lane] = hit ? r2 : T(0);
+            W.rz[b][lane] = hit ? p.a2 * r2 : T(0);
         }
     };
     if (p.comp) fill([&](int g, T yy) { return fma_t((T)g, p.h_hi, -yy) + (T)g * p.h_lo; });
@@ -433,7 +438,7 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 10 : 6)
             load_pairs<T, MGT>(&W.wx[e][0], w);
 #pragma unroll
             for (int k = 0; k < MGT / 2; ++k) {
-                const pair2<T> wgt = fma2(w[k], g2, mul2(w[MGT / 2 + k], q2));
+                const pair2<T> wgt = mul2(w[k], fma2(w[MGT / 2 + k], g2, q2));
 #pragma unroll
                 for (int c = 0; c < 3; ++c) acc[c][k] = fma2(wgt, f[c], acc[c][k]);
             }
@@ -550,7 +555,7 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 8 : 5)
                 pair2<T> v[3];
 #pragma unroll
                 for (int k = 0; k < MGT / 2; ++k) {
-                    const pair2<T> wgt = fma2(w[k], g2, mul2(w[MGT / 2 + k], q2));
+                    const pair2<T> wgt = mul2(w[k], fma2(w[MGT / 2 + k], g2, q2));
 #pragma unroll
                     for (int c = 0; c < 3; ++c) v[c] = k == 0 ? mul2(wgt, u[c][0]) : fma2(wgt, u[c][k], v[c]);
                 }
@@ -559,10 +564,12 @@ __global__ void __launch_bounds__(32 * PENCIL_WARPS, sizeof(T) == 4 ? 8 : 5)
             }
             __syncwarp();
             if (lane < 3 * m) {
-                T v = 0;
+                // in eight partial sums, then pairwise
+                T v[8];
 #pragma unroll
-                for (int r = 0; r < 32; ++r) v += I.part[lane][r];
-                atomicAdd(Vs + 3 * (int64_t)I.s[e0 + lane / 3] + lane % 3, v);
+                for (int r = 0; r < 32; ++r) v[r % 8] = r < 8 ? I.part[lane][r] : v[r % 8] + I.part[lane][r];
+                atomicAdd(Vs + 3 * (int64_t)I.s[e0 + lane / 3] + lane % 3,
+                          ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
             }
             __syncwarp();
         }
