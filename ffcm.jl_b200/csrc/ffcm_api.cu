@@ -1313,17 +1313,28 @@ struct Engine final : EngineBase {
 
     // Whether the pencil kernels beat one warp per particle (global atomics in
     // the spread). Their cost grows with the pencils a particle reaches and, as
-    // every pencil is walked whether or not it holds particles, with the grid;
-    // the lists are three more launches. Spread + interpolation, warp per
-    // particle against pencils, by stencil points N M_G^3 and their ratio to the
-    // grid's points: 187M, 11: 1458 / 687 us (Float64 1822 / 1191); 86M, 2.6:
-    // 695 / 557; 43M, 1.3 (Float64): 838 / 876; 23M, 3.3: 191 / 192 (Float64
-    // 274 / 314, whose pencils keep fewer warps on an SM); 15M, 7: 130 / 137;
-    // 15M, 1.9: 144 / 193. FFCM_PENCIL = 0 or 1 forces the choice.
+    // every pencil is walked whether or not it holds particles, with the grid,
+    // more so where rows do not start on 32-byte sectors; the lists are three
+    // more launches. Spread + interpolation, warp per particle against pencils,
+    // by stencil points N M_G^3, their ratio to the grid's points and M_G:
+    //  * whole sectors, Float32: 187M, 11, 10: 1379 / 612 us; 60M, 3.6, 10: 487 /
+    //    326; 44M, 2.6, 9: 362 / 308; 24M, 3, 10: 217 / 194; but 22M, 2.8, 7: 203
+    //    / 224; 21M, 2.7, 8: 178 / 186; 16M, 11, 12: 131 / 137; 41M, 2.3, 7: 387 / 463
+    //  * whole sectors, Float64: 187M, 11, 10: 1809 / 1055; 66M, 2.7, 9: 790 /
+    //    654; 52M, 3.1, 7: 659 / 620; but 52M, 2.9, 7: 669 / 732; below 5e7 points
+    //    44M, 5.7, 9: 464 / 398, but 26M, 3.2, 6: 362 / 400 and 16M, 11, 12: 168 / 188
+    //  * other rows, Float32: 60M, 3.8, 10: 487 / 445; 32M, 3.5, 6: 306 / 280; 26M,
+    //    3.8, 8: 209 / 207; but 36M, 3.2, 9: 295 / 327; 45M, 2.9, 10: 384 / 431;
+    //    Float64: 60M, 3.8, 10: 658 / 566; 58M, 5.1, 9: 616 / 553; but 56M, 3.6, 8:
+    //    625 / 736; 65M, 4.1, 6: 847 / 877
+    // FFCM_PENCIL = 0 or 1 forces the choice.
     bool pencil_pays() const {
         if (const char* v = std::getenv("FFCM_PENCIL")) return v[0] == '1';
+        const bool f32 = sizeof(T) == 4;
         const double points = (double)N * MG * MG * MG;
-        return points >= (sizeof(T) == 4 ? 2e7 : 5e7) && points >= 2.5 * (double)plane;
+        double ratio = (f32 ? points < 3e7 : MG < 8) ? 3.0 : 2.5;
+        if (Mx * sizeof(T) % 32 != 0) ratio = f32 ? 3.4 : MG >= 10 ? 3.5 : 4.0;
+        return points >= (f32 ? 2e7 : 5e7) && points >= ratio * (double)plane;
     }
 
     // The pencils' particle lists of the sorted positions.
