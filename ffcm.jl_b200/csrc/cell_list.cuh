@@ -149,9 +149,9 @@ __global__ void k_scan_apply(const int32_t* __restrict__ count, int n,
 
 // The whole scan in one launch for up to SCAN_ONE_PASS counts: every block adds
 // up all counts before its tile itself. What it reads grows with the square of
-// the tiles: 4.4 us at 2,197 cells and 12.5 us at 64,000, where the three
-// launches above take 15 us.
-constexpr int SCAN_ONE_PASS = 1 << 15;
+// the tiles. The cell list, one launch against the three above: 46,656 cells 29.0 /
+// 32.5 us, 64,000 30.4 / 31.2, 85,184 32.3 / 32.1, 125,000 36.4 / 32.3.
+constexpr int SCAN_ONE_PASS = 1 << 16;
 
 __global__ void k_scan_one_pass(const int32_t* __restrict__ count, int n, int32_t* __restrict__ off) {
     __shared__ int smem[32];

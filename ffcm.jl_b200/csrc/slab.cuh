@@ -70,8 +70,10 @@ struct SlabShape {
 // so a further block per SM is worth some spilled registers wherever shared
 // memory holds it. 256^3, N = 60,000, us by blocks: Float32 spread 203 (3), 183
 // (4), 204 (5), interpolation 172 (3), 155 (4), 147 (5), 156 (6); Float64 spread 568 (2),
-// 457 (3), 413 (4), interpolation 470 (2), 385 (3), 374 (4); and the 512 slabs
-// of a 64^3 grid run at once. From x length 512 on shared memory decides.
+// 457 (3), 413 (4). Float64 interpolation, whose fourth block spills 500 bytes a
+// thread, 3 against 4 blocks: 396 / 360 (N = 62,500) and 376 / 333 (20,000), at
+// 128^3 90 / 86 (30,000) and 73 / 62 (8,000), at 64^3 25.0 / 21.0 (2,000). The 512
+// slabs of a 64^3 grid run at once. From x length 512 on shared memory decides.
 template <typename T, int H>
 constexpr int spread_blocks() { return H <= 128 ? 4 : sizeof(T) == 8 ? 2 : 3; }
 template <typename T, int H>

@@ -50,3 +50,13 @@ def test_slab_lists_over_many_cell_rows(ffcm, T):
     # 12 x 10 cell rows reach a slab of 4 x 2 grid rows
     _, _, V, ref, _, _ = _solve_twice(ffcm, T, kw_of(64.0, 3000, 64, R_c=1.0), 7)
     assert rel_l2(V, ref) < TOL[T]
+
+
+@pytest.mark.parametrize("cells", [(64, 32, 32), (41, 40, 40)])
+def test_cell_list_scan_limit(ffcm, cells):
+    """65,536 cells (one launch) and 65,600 (three)."""
+    kw = kw_of(tuple(float(c) for c in cells), 4000, cells, M_G=4, R_c=1.0)
+    prod, ora, V, ref, Y, F = _solve_twice(ffcm, np.float64, kw, sum(cells))
+    assert np.array_equal(prod.original_index, ora.original_index)
+    assert np.array_equal(prod.cell_start, ora.cell_start) and np.array_equal(prod.cell_end, ora.cell_end)
+    assert rel_l2(V, ref) < TOL[np.float64]
