@@ -197,7 +197,10 @@ int derive_T(const double* Ld, double R_cd, double ad, double ratiod, const int3
 // product of register butterflies and single primes up to MIX_MAX_PRIME, by a
 // model of a stage's cost per value fitted to measured passes (y pass of 240 x
 // 200 x 160 in Float32: radices 20 10: 55 us, 8 5 5: 63, 25 8: 74, 10 5 4: 84;
-// z pass: 16 10: 78, 20 8: 85, 10 4 4: 115). Largest radix first, so that the last
+// z pass: 16 10: 78, 20 8: 85, 10 4 4: 115). Float64, with the same costs and its
+// own radices: within 5% of the fastest plan of all lengths tried on the y and z
+// axes (105 to 300; y of 240: 16 15 70 us, 12 5 4: 89; z of 240: 8 6 5 169, 10 6
+// 4: 161; z of 108: 6 6 3 68, 12 9: 75). Largest radix first, so that the last
 // one is the smallest. max_last > 0: also the cheapest plan whose last radix
 // is at most max_last, taken when it has no more than one stage more (the z
 // pass then keeps a fused projector stage in registers).
@@ -1363,7 +1366,7 @@ struct Engine final : EngineBase {
                       (const int*)pen_off, (const int*)pen_ent, pen_tasks, gf, partial, 3 * (int64_t)N);
     }
 
-    // velocities gu -> h^-3 V in sorted order in `partial`
+    // velocities gu -> h^-3 V in sorted order added to `partial` (zeroed by the spread)
     int pencil_interp(cudaStream_t s) {
         StageScope sc(h, FFCM_STAGE_INTERPOLATE, s);
         return launch(h, pk.interp, pencil_blocks(), 32 * PENCIL_WARPS, pk.smem_interp, s, (const vec4<T>*)Ys, sp, pg,
@@ -1418,7 +1421,8 @@ struct Engine final : EngineBase {
         return launch_y(s, 1);
     }
 
-    // x-c2r + gather; leaves h^-3 V in sorted order in `partial` for correct_final.
+    // x-c2r + gather; adds h^-3 V in sorted order to `partial`, which a spread of
+    // this solve has zeroed (every caller without one zeroes it), for the correction.
     int interp_from_spectrum(cudaStream_t s) {
         StageScope sc(h, FFCM_STAGE_INTERPOLATE, s);
         dim3 g(sg.nty, sg.ntz, 1);
@@ -1526,9 +1530,12 @@ struct Engine final : EngineBase {
     // with events around its y forward pass and its correction, and a later
     // solve, once those have completed, fixes the mode for the configuration:
     // overlap when the correction took under half the y pass and the y pass over
-    // 0.4 ms (a short y pass ends before the correction, whose blocks then delay
-    // the z pass's single wave: 256^3 Float64, N = 62,500: 1641 us on one
-    // stream, 1690 us overlapped; Float32 732 / 736). `side` tells
+    // 0.4 ms (after a shorter one the correction's blocks can delay the z pass's
+    // single wave; one stream / overlapped, us by the y pass: 157 us, 256^3
+    // Float64, N = 62,500: 1382 / 1437; 304 us, 512 x 256 x 512: 2392 / 2680; 318
+    // us, 512 x 512 x 256: 2504 / 2454; 617 us, 512^3, N = 500,000: 4789 / 4712).
+    // Eight configurations made one after the other, and further ones in fresh
+    // processes, all took the same order. `side` tells
     // the caller whether it forked, `probe` whether to record the events
     // (ev_probe[0..1] around the y forward pass, [2..3] around k_correct).
     // Under capture (the batched graph, the CG loop) the solve keeps the

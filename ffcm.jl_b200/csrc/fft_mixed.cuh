@@ -317,7 +317,7 @@ __device__ __forceinline__ void mix_run_stage(const MixPlan& p, int s, int Ns, i
 // The twiddle table W_n^e of the axis (`count` values): from shared memory at
 // `sm`, where the block starts copying it, or from global memory (LONG).
 template <typename T, bool LONG>
-__device__ __forceinline__ const cplx<T>* mix_table(cplx<T>* sm, const cplx<T>* __restrict__ table, int count) {
+__device__ __forceinline__ const cplx<T>* mix_twiddles(cplx<T>* sm, const cplx<T>* __restrict__ table, int count) {
     if constexpr (LONG) {
         return table;
     } else {
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256)
     cplx<T>* sm = reinterpret_cast<cplx<T>*>(smem_raw);
     const int n = p.n;
     MixBuf<T> cur{LONG ? sm : sm + n, 1 << lb, 0}, other{cur.p + (n << lb), 1 << lb, 0};
-    const cplx<T>* tw = mix_table<T, LONG>(sm, table, n);
+    const cplx<T>* tw = mix_twiddles<T, LONG>(sm, table, n);
     // whole tiles: the row pitch is a multiple of the tile width, the padding
     // columns hold whatever they held, transformed
     const MixSpan<T> g{spec + ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * n * hxp + (blockIdx.x << lb), hxp, 0};
@@ -449,7 +449,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256, sizeof(T) == 4 ? 1
     const int n = p.n, cs = n << lb;
     cplx<T>* sm = reinterpret_cast<cplx<T>*>(smem_raw);
     MixBuf<T> cur{LONG ? sm : sm + n, 1 << lb, cs}, other{cur.p + 3 * cs, 1 << lb, cs};
-    const cplx<T>* tw = mix_table<T, LONG>(sm, table, n);
+    const cplx<T>* tw = mix_twiddles<T, LONG>(sm, table, n);
     const int kx0 = blockIdx.x << lb, y = blockIdx.y;
     const int64_t zs = (int64_t)My * hxp;
     const MixSpan<T> g{spec + (int64_t)y * hxp + kx0, zs, n * zs};
@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256)
     const int n = p.n, pitch = lb ? (1 << lb) + 1 : 1;
     cplx<T>* sm = reinterpret_cast<cplx<T>*>(smem_raw);
     cplx<T>* A = LONG ? sm : sm + Mx;
-    const cplx<T>* tw = mix_table<T, LONG>(sm, table, Mx);
+    const cplx<T>* tw = mix_twiddles<T, LONG>(sm, table, Mx);
     const bool even = (Mx & 1) == 0;
     const int per = even ? 1 : 2, nlines = (nrows + per - 1) / per;
     const int line0 = blockIdx.x << lb, nl = min(1 << lb, nlines - line0);
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 512 : 256)
     const int n = p.n, pitch = lb ? (1 << lb) + 1 : 1;
     cplx<T>* sm = reinterpret_cast<cplx<T>*>(smem_raw);
     cplx<T>* A = LONG ? sm : sm + Mx;
-    const cplx<T>* tw = mix_table<T, LONG>(sm, table, Mx);
+    const cplx<T>* tw = mix_twiddles<T, LONG>(sm, table, Mx);
     const bool even = (Mx & 1) == 0;
     const int per = even ? 1 : 2, nlines = (nrows + per - 1) / per;
     const int line0 = blockIdx.x << lb, nl = min(1 << lb, nlines - line0);

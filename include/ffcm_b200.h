@@ -27,8 +27,14 @@
  *    `stream` is being captured into a CUDA graph), so the call stays
  *    ordered on `stream` as a whole. A handle's first solve times its
  *    correction against its y pass and later solves fork only when the
- *    correction is the shorter by half; FFCM_OVERLAP_PAIRS=0 (never) or 1
- *    (always) in the environment at ffcm_create overrides that.
+ *    correction is the shorter by half and the y pass over 0.4 ms;
+ *    FFCM_OVERLAP_PAIRS=0 (never) or 1 (always) in the environment at
+ *    ffcm_create overrides that.
+ *  - Where the fused slab kernels do not apply (M_G != 8 or a grid that is no
+ *    power of two along x), FFCM_PENCIL=0 or 1 in the environment at
+ *    ffcm_create keeps the assembled solve on the warp-per-particle spread and
+ *    interpolation or puts it on the pencil kernels (M_G up to 12), which are
+ *    otherwise chosen by the numbers of particles and grid points.
  *  - Index buffers exchanged through ffcm_get_buffer/ffcm_set_buffer are
  *    1-based, as in the reference (`original_index`, `cell_start`,
  *    `cell_end`); cell hashes are 0-based as in the reference.

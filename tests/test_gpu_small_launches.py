@@ -20,7 +20,9 @@ def _solve_twice(ffcm, T, kw, seed):
         Y = (rng.random((kw["N"], 3)) * np.array(kw["L"])).astype(T)
         F = rng.standard_normal((kw["N"], 3)).astype(T)
         V = ffcm.mobility(np.empty_like(Y), prod, Y, F)
-    return prod, ora, V, O.apply(ora, Y, F), Y, F
+        ref = O.apply(ora, Y, F)
+        assert rel_l2(V, ref) < TOL[np.dtype(T).type]
+    return prod, ora, V, ref, Y, F
 
 
 @pytest.mark.parametrize("cells", [(3, 3, 3), (16, 16, 8), (32, 32, 32), (33, 32, 32), (40, 41, 42)])
