@@ -25,14 +25,14 @@
 // configuration (N = 186,510) are 2.49e-7 off in Float32 (mean of five seeds)
 // against 2.34e-7 with a warp per particle, in Float64 5.34e-16 against 5.13e-16.
 //
-// What bounds it: instruction issue (ncu: 66% of issue slots, the rest waits on
+// What bounds it: instruction issue (ncu: 63% of issue slots, the rest waits on
 // shared memory): per entry and pencil 2.5 M_G two-wide multiply-adds and as
 // many instructions again for its weights, loads and the walk; of the
 // (M_G + 7)(M_G + 3) rows its pencils hold, an entry uses M_G^2. N = 186,510,
-// 256^3, M_G = 10, Float32: spread 300 us (the lists 35 us more) against 700 us
+// 256^3, M_G = 10, Float32: spread 296 us (lists and zeroing 39 us more) against 700 us
 // with global atomics, which run at one 32-byte sector per L2 slice and clock;
 // interpolation 273 against 675 us, where every warp read 20 KB through L1
-// (Float64: 475 and 534 against 1035 and 775 us).
+// (Float64: 470 and 534 against 1035 and 775 us).
 #pragma once
 
 #include "common.cuh"
@@ -310,8 +310,9 @@ struct PencilRows {
             for (int b = 0; b < PENCIL_TY; b += GROUP)
                 f(d * PENCIL_TY + b + lane / XC, b < ny && d < nz, base + d * zs + b * p.Mx);
     }
-    // staged columns added to the grid, where `on` (rolled: the code of 96 atomics
-    // beside the stores cost every spread a tenth of its time)
+    // staged columns added to the grid, where `on` (rolled: with the code of 96
+    // atomics beside the stores, and a third more idle blocks, every spread of the
+    // record configuration took 371 us instead of 335)
     __device__ __forceinline__ void add(const StencilParams<T>& p, int lane, bool on, int64_t plane, T* out,
                                      const T (*stage)[32][XC + 1]) const {
         if (!on) return;
