@@ -912,23 +912,27 @@ struct Engine final : EngineBase {
         TRY(alloc(kyv, My));
         TRY(alloc(kzv, Mz));
         if (slab) {
-            TRY(alloc(partial, 3 * (size_t)N));
+            // (the pair terms too: the first overlapped solve, some solves after
+            // the first, does not wait for an allocation)
+            TRY(alloc(partial, 6 * (size_t)N));
+            dvs = partial + 3 * (size_t)N;
             TRY(alloc(slab_lists, (size_t)sg.nty * sg.ntz * sg.lcap));
             TRY(alloc(slab_counts, (size_t)sg.nty * sg.ntz));
         }
 
         if (pencil) {
-            // one allocation (each costs 0.2 to 0.3 ms): interpolation sums, then
+            // one allocation (each costs 0.2 to 0.3 ms): interpolation sums, pair terms, then
             // further parts, counts, entries used and parts used, offsets, parts, entries
             const size_t noff = (size_t)pen_bins + (size_t)pg.nty * pg.ntz;
             const size_t nent = (size_t)N * pencil_reach(PENCIL_TY, MG, My) * pencil_reach(PENCIL_TZ, MG, Mz);
             // an entry's stencil lies in two segments, or three with a short last one
             pen_more = (int)((pg.nseg == 1 || Mx % pg.seg == 0 ? 2 : 3) * nent / pg.part) + 1;
             const size_t nseg = (size_t)pg.nty * pg.ntz * pg.nseg;
-            const size_t sums = (3 * (size_t)N * sizeof(T) + 15) / 16 * 16, more = (size_t)pen_more * sizeof(int2);
+            const size_t sums = (6 * (size_t)N * sizeof(T) + 15) / 16 * 16, more = (size_t)pen_more * sizeof(int2);
             unsigned char* base = nullptr;
             TRY(alloc(base, sums + more + ((size_t)pen_bins + 2 + noff + nseg + nent) * sizeof(int)));
             partial = reinterpret_cast<T*>(base);
+            dvs = partial + 3 * (size_t)N;
             pen_tasks.more = reinterpret_cast<int2*>(base + sums);
             pen_cnt = reinterpret_cast<int*>(base + sums + more);
             pen_used = pen_cnt + pen_bins;
@@ -1575,7 +1579,6 @@ struct Engine final : EngineBase {
             }
             if (!h->pair_overlap) return FFCM_OK;
         }
-        if (!dvs) TRY(alloc(dvs, 3 * (size_t)N));
         if (!h->side_stream) {
             CUDA_TRY(cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking));
             CUDA_TRY(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));

@@ -78,3 +78,28 @@ def test_first_gradient_and_cg(ffcm, busy, T, M, MG):
     first = ffcm.cg(A, F, reltol=0.0, maxiter=4)
     again = ffcm.cg(A, F, reltol=0.0, maxiter=4)
     assert rel_l2(first, again) < TOL[T]
+
+
+def test_overlapped_solve_allocates_nothing(ffcm, monkeypatch):
+    """The first solve with the correction on the side stream, which a
+    configuration takes some solves after its first, works in memory from the
+    configuration's creation."""
+    import torch
+    monkeypatch.setenv("FFCM_OVERLAP_PAIRS", "1")
+    N, M = 1_000_000, 256
+    L = (0.9 * M,) * 3
+    g = torch.Generator("cuda")
+    g.manual_seed(4)
+    Y = torch.rand(N, 3, generator=g, device="cuda") * L[0]
+    F = torch.randn(N, 3, generator=g, device="cuda")
+    V = torch.empty_like(F)
+    kw = kw_of(L, N, M, R_c=3.0)
+    warm = ffcm.FFCMConfig(np.float32, **kw)      # loads the kernels
+    ffcm.mobility(V, warm, Y, F)
+    cfg = ffcm.FFCMConfig(np.float32, **kw)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    ffcm.mobility(V, cfg, Y, F)
+    torch.cuda.synchronize()
+    # (the pair terms of N particles are 12 MB; streams and events take some room)
+    assert before - torch.cuda.mem_get_info()[0] < 8 << 20
